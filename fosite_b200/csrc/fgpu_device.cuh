@@ -182,6 +182,37 @@ __device__ __forceinline__ double dmin(double a, double b) { return fmin(a, b); 
 __device__ __forceinline__ double dmax(double a, double b) { return fmax(a, b); }
 #endif
 
+// ---------------------------------------------------------------- reciprocals
+#ifndef FGPU_EXACT
+// Reciprocal and reciprocal square root of the product build.  The hardware's approximations
+// (rcp/rsqrt.approx.ftz.f64) are refined by one step of Householder's cubic iteration
+// (1/d: y + y (e + e^2) with e = 1 - d y; 1/sqrt(q): y + y (e/2 + 3 e^2/8) with e = 1 - q y^2),
+// which cubes the relative error.  Straight-line code: the compiler's division and square root
+// carry a branch to a slow path at every use, and the stage kernels hold up to twenty of them.
+// d and q must be normal, finite and not within a factor 2^2 of the range's ends (in_range);
+// 0, infinities and NaN give NaN.  Measured over 12.6 million values of exponents -950 to 950 the
+// largest relative errors are 1.00 (reciprocal) and 1.25 (square root) times 2^-53; with the
+// selections of the limiters and wave speeds below the 256^3 Dormand-Prince step went from
+// 17.0 to 14.2 ms, the 2D boxes' steps by 4 to 11%.
+__device__ __forceinline__ double rcp_refined(double d) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+  const double e = fma(-d, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+__device__ __forceinline__ double rsqrt_refined(double q) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(q));
+  const double e = fma(-q * y, y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
+// 2^-LO <= x < 2^HI (x positive), by its exponent: one integer subtraction and comparison
+template <int LO, int HI>
+__device__ __forceinline__ bool in_range(double x) {
+  return (unsigned)(__double2hiint(x) - ((1023 - LO) << 20)) < (unsigned)((HI + LO) << 20);
+}
+#endif
+
 // ---------------------------------------------------------------- physics
 // Variables: 0 density, 1..ND velocity/momentum, ND+1 pressure/energy (Euler).
 template <int ND, bool EU>
@@ -190,7 +221,12 @@ struct Phys {
 
   // Cons2Prim (physics_euler.f90:3064-3100, physics_eulerisotherm.f90:2831-2856)
   static __device__ __forceinline__ void c2p(const double* c, double* p, const PhysP& P) {
+#ifdef FGPU_EXACT
     double inv_rho = 1. / c[0];
+#else
+    double inv_rho = rcp_refined(c[0]);
+    if (!in_range<1000, 1000>(c[0])) inv_rho = 1. / c[0];   // zero, negative, extreme or NaN densities
+#endif
     p[0] = c[0];
 #pragma unroll
     for (int m = 1; m <= ND; ++m) p[m] = c[m] * inv_rho;
@@ -216,21 +252,29 @@ struct Phys {
     }
   }
   // GetSoundSpeed (physics_euler.f90:2682-2689): sqrt(MAX(2 TINY, gamma*p/rho)).
-  // The product build evaluates sqrt(s/rho) as s*rsqrt(s*rho) with s = gamma*p (one
-  // reciprocal square root instead of a division and a square root; within a few ulp).
+  // The product build evaluates sqrt(s/rho) as s*rsqrt(s*rho) with s = gamma*p (within a few
+  // ulp); the range test keeps s*rho and s/rho away from the ends of the double range, where
+  // the reference's form takes over.
   static __device__ __forceinline__ double cs_of(const double* p, const PhysP& P) {
 #ifdef FGPU_EXACT
     return sqrt(dmax(P.tiny2, P.gamma * p[V - 1] / p[0]));
 #else
     const double s = P.gamma * p[V - 1];
-    const double q = s * p[0];
-    if (s > P.tiny2 * p[0] && q > 1e-300 && q < 1e300) return s * rsqrt(q);
+    if (in_range<480, 480>(s) && in_range<480, 480>(p[0])) return s * rsqrt_refined(s * p[0]);
     return sqrt(dmax(P.tiny2, s / p[0]));
 #endif
   }
 };
 
 // ---------------------------------------------------------------- limiters
+#ifndef FGPU_EXACT
+// the smaller in magnitude of two differences of one sign, else zero: one FP64 comparison, the
+// sign test on the high words
+__device__ __forceinline__ double minmod2(double a, double b) {
+  const double m = fabs(b) < fabs(a) ? b : a;
+  return (__double2hiint(a) ^ __double2hiint(b)) < 0 ? 0.0 : m;
+}
+#endif
 // reconstruction_linear.f90:645-733; returns the limited difference (times invd by caller)
 __device__ __forceinline__ double limit2(int lim, double theta, double a1, double a2) {
   switch (lim) {
@@ -239,9 +283,7 @@ __device__ __forceinline__ double limit2(int lim, double theta, double a1, doubl
       if (fsign1(a1) * fsign1(a2) > 0) return fsign(dmin(fabs(a1), fabs(a2)), a1);
       return 0.;
 #else
-      // the same value for non-zero differences (see MONOCENT in slope)
-      const double lo = dmin(a1, a2), hi = dmax(a1, a2);
-      return lo > 0. ? lo : (hi < 0. ? hi : 0.);
+      return minmod2(a1, a2);
 #endif
     }
     case LIM_SWEBY:
@@ -255,7 +297,13 @@ __device__ __forceinline__ double limit2(int lim, double theta, double a1, doubl
       return 1.5 * a1 * a2 * (a1 + a2) / (a1 * (a1 + 0.5 * a2) + a2 * (a2 + 0.5 * a1) + DBL_MIN);
     case LIM_VANLEER: {
       double b1 = fabs(a1), b2 = fabs(a2);
+#ifdef FGPU_EXACT
       return (a1 * b2 + a2 * b1) / (b1 + b2 + DBL_MIN);
+#else
+      // the denominator is at least DBL_MIN, whose reciprocal is in range; one that overflows
+      // goes with a numerator that has overflowed already
+      return (a1 * b2 + a2 * b1) * rcp_refined(b1 + b2 + DBL_MIN);
+#endif
     }
     case LIM_NOLIMIT:
       return 0.5 * (a1 + a2);
@@ -265,19 +313,19 @@ __device__ __forceinline__ double limit2(int lim, double theta, double a1, doubl
 }
 // slope of q0 with neighbours qm, qp (MONOCENT uses minmod3 of three differences)
 __device__ __forceinline__ double slope(int lim, double theta, double invd, double qm, double q0, double qp) {
-  if (lim == LIM_MC || lim == LIM_MC1) {
-    double a1 = lim == LIM_MC1 ? q0 - qm : theta * (q0 - qm), a2 = lim == LIM_MC1 ? qp - q0 : theta * (qp - q0);
+  // MC with theta = 1 is minmod: the central difference is the mean of the one-sided ones, and
+  // rounding is monotonic, so (qp - qm)/2 is never the smallest of the three in magnitude
+  if (lim == LIM_MC1) return invd * limit2(LIM_MINMOD, theta, q0 - qm, qp - q0);
+  if (lim == LIM_MC) {
+    double a1 = theta * (q0 - qm), a2 = theta * (qp - q0);
     double a3 = 0.5 * (qp - qm);
 #ifdef FGPU_EXACT
     double r = 0.;
     if (((fsign1(a1) * fsign1(a2)) > 0) && ((fsign1(a2) * fsign1(a3)) > 0))
       r = fsign(dmin(dmin(fabs(a1), fabs(a2)), fabs(a3)), a1);
 #else
-    // same value as the sign-test form for all non-zero slopes: the smallest of three
-    // positive differences, the largest of three negative ones, else zero (the sign of
-    // a zero result may differ)
-    const double lo = dmin(dmin(a1, a2), a3), hi = dmax(dmax(a1, a2), a3);
-    const double r = lo > 0. ? lo : (hi < 0. ? hi : 0.);
+    // the smallest in magnitude of three differences of one sign, else zero
+    const double r = minmod2(minmod2(a1, a2), a3);
 #endif
     return invd * r;
   }
@@ -562,10 +610,13 @@ __device__ __forceinline__ void kt_flux(int d_rt, const double* RL, const double
   double am = dmin(dmin(0.0, dmin(0., uR - csR)), dmin(0., uL - csL));
   double ap = dmax(dmax(0.0, dmax(0., uR + csR)), dmax(0., uL + csL));
 #else
-  // the same extrema with two native min/max each (a zero result may differ in sign, which
-  // no flux component sees: it enters as a product and in ap - am)
-  double am = dmin(0.0, dmin(uR - csR, uL - csL));
-  double ap = dmax(0.0, dmax(uR + csR, uL + csL));
+  // the same extrema by comparison and selection, the clip at zero by the sign bit (a zero
+  // result may differ in sign, which no flux component sees: it enters as a product and in
+  // ap - am); a NaN wave speed stays NaN in the flux through the face's own states
+  const double mR = uR - csR, mL = uL - csL, qR = uR + csR, qL = uL + csL;
+  double am = mR < mL ? mR : mL, ap = qR > qL ? qR : qL;
+  am = __double2hiint(am) < 0 ? am : 0.0;
+  ap = __double2hiint(ap) < 0 ? 0.0 : ap;
 #endif
   double fL[V], fR[V];
   fL[0] = pL[0] * uL;
@@ -586,7 +637,11 @@ __device__ __forceinline__ void kt_flux(int d_rt, const double* RL, const double
       fR[m] = (m == vn) ? cR[m] * uR + pR[0] * csR * csR : cR[m] * uR;
     }
   }
+#ifdef FGPU_EXACT
   double fac = dA / (ap - am);
+#else
+  double fac = dA * rcp_refined(ap - am);
+#endif
   double amap = am * ap;
 #pragma unroll
   for (int l = 0; l < V; ++l) F[l] = fac * (ap * fL[l] - am * fR[l] + amap * (cR[l] - cL[l]));
