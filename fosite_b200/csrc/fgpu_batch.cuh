@@ -16,13 +16,23 @@ struct fgpu_batch {
   int nd = 2, order = 3;
   bool euler = false, prim = false;
   cudaStream_t stream = nullptr;
-  int variant = 0;               // stage layout: 0/2/3 shared-memory tiles, 6 TMA-staged tiles (2D)
+  int variant = 0;               // stage layout: 0/6 the marching kernels (0: the base tile where they do
+                                 // not serve the batch), 2/3 shared-memory tiles
   StageArgs* d_args = nullptr;   // [order][n] step stages, then [n] RHS probes of the tuner
-  CUtensorMap* d_maps = nullptr; // [order + 1][n] tensor maps of the stage inputs of d_args (layout 6)
-  int tma_lim = -1;              // compiled-in limiter of layout 6, -1 when the batch cannot use it
-  int4* d_tcols = nullptr;       // layout 6: (member, bx, byb, 0), columns of kchunk tiles per block
-  int ntcols = 0;
-  std::vector<char> tma_red;     // layout 6: per row of d_args, whether some member's stage reduces
+  // marching layout: whether every stage of the batch can use it, the compiled-in limiter, the
+  // block queue (2D: (member, first warp, has a tensor map, 0); 3D: (member, bx, by, bz)), rows per
+  // warp (2D), and per argument table the tensor maps of the stage inputs, whether some member's
+  // stage of a row reduces and whether every member's is a plain_stage
+  bool march = false;
+  int march_lim = 0;
+  int4* d_mqueue = nullptr;
+  int nmqueue = 0;
+  int march_rows = 0;
+  struct MarchTable {
+    CUtensorMap* d_maps = nullptr;
+    std::vector<char> red, plain;
+  };
+  MarchTable march_args, march_eargs;   // of d_args, d_eargs
   BndArgs* d_bnd = nullptr;      // [n]
   int4* d_tiles = nullptr;
   int ntiles = 0;
@@ -76,15 +86,25 @@ int bset_err(fgpu_batch* b, int code, const std::string& msg) {
                       std::string(#call) + ": " + cudaGetErrorString(e_));                   \
   } while (0)
 
+bool in_table(const StageArgs* args, const StageArgs* t, size_t n) { return t && args >= t && args < t + n; }
+
 int launch_batched_stage(fgpu_batch* b, const StageArgs* args, int variant) {
-  if (variant == 6) {   // TMA-staged tiles: tensor maps parallel to the step and probe tables
-    if (!b->d_maps || args < b->d_args || args >= b->d_args + (size_t)(b->order + 1) * b->m.size())
-      return bset_err(b, FGPU_EUNSUPPORTED, "the TMA layout serves fixed-step 2D batches only");
-    const size_t row = (size_t)(args - b->d_args) / b->m.size();
-    BCUDA_TRY(b, tma_batched_launch_2d(b->euler, b->prim, b->tma_lim, b->tma_red[row] != 0, args,
-                                       b->d_maps + (args - b->d_args), b->d_tcols, b->ntcols, b->stream));
+  if ((variant == 0 || variant == 6) && b->march) {
+    const size_t n = b->m.size();
+    const bool e = in_table(args, b->d_eargs, (size_t)(b->stages + 2) * n);
+    const fgpu_batch::MarchTable& T = e ? b->march_eargs : b->march_args;
+    const size_t at = (size_t)(args - (e ? b->d_eargs : b->d_args)), row = at / n;
+    const bool red = T.red[row] != 0, plain = T.plain[row] != 0;
+    const CUtensorMap* maps = T.d_maps + at;
+    if (b->nd == 2)
+      BCUDA_TRY(b, (b->euler ? strip2_batch_launch_euler : strip2_batch_launch_iso)(
+                       b->prim, b->march_lim, red, plain, args, maps, b->d_mqueue, b->nmqueue, b->stream));
+    else
+      BCUDA_TRY(b, (b->euler ? march3_batch_launch_euler : march3_batch_launch_iso)(
+                       b->prim, b->march_lim, red, plain, args, maps, b->d_mqueue, b->nmqueue, b->stream));
     return FGPU_OK;
   }
+  if (variant == 6) variant = 0;
   // the shared-memory base tile of the batch's tile queue: layouts 0, 2, 3
   if (b->nd == 2)
     BCUDA_TRY(b, legacy_batched_launch_2d(b->euler, b->prim, variant, args, b->d_tiles, b->ntiles, b->sms, b->stream));
@@ -192,6 +212,33 @@ int upload_table(fgpu_batch* b, T** dst, const std::vector<T>& v) {
   BCUDA_TRY(b, cudaMalloc(dst, sizeof(T) * std::max<size_t>(1, v.size())));
   BCUDA_TRY(b, cudaMemcpyAsync(*dst, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, b->stream));
   return FGPU_OK;
+}
+
+// The marching layout's tables of rows of stage arguments (one entry per member and row): tensor
+// maps of the stage inputs, the kernel forms of each row; 2D arguments get the rows per warp.
+// Clears b->march when a member's stage cannot use the layout.
+int build_march_table(fgpu_batch* b, std::vector<StageArgs>& args, fgpu_batch::MarchTable& T) {
+  const size_t n = b->m.size(), rows = args.size() / n;
+  std::vector<CUtensorMap> maps(args.size());
+  std::memset(maps.data(), 0, sizeof(CUtensorMap) * maps.size());
+  T.red.assign(rows, 0);
+  T.plain.assign(rows, 1);
+  for (size_t q = 0; q < args.size() && b->march; ++q) {
+    fgpu_handle* h = b->m[q % n];
+    const StageArgs& A = args[q];
+    if (!tma_eligible(h, A)) b->march = false;
+    if (b->march && stage_has_tmap(h)) {
+      const CUtensorMap* mp = stage_tmap(h, A.rin.base ? A.rin.base : A.in.base);
+      if (mp) maps[q] = *mp;
+      else b->march = false;
+    }
+    if (A.cfl_mode || A.last_stage || A.err_low) T.red[q / n] = 1;
+    if (!plain_stage(A)) T.plain[q / n] = 0;
+  }
+  if (!b->march) return FGPU_OK;
+  if (b->nd == 2)
+    for (auto& A : args) A.kchunk = b->march_rows;
+  return upload_table(b, &T.d_maps, maps);
 }
 
 // The argument tables of the attempt slot: what enqueue_bt_slot launches for one grid,
@@ -305,6 +352,8 @@ int build_embedded_tables(fgpu_batch* b) {
   b->ncblocks = (int)cblocks.size();
   if (int rc = upload_table(b, &b->d_ctlp, ctlp)) return rc;
   if (int rc = upload_table(b, &b->d_btp, btp)) return rc;
+  if (b->march)
+    if (int rc = build_march_table(b, eargs, b->march_eargs)) return rc;
   if (int rc = upload_table(b, &b->d_eargs, eargs)) return rc;
   if (int rc = upload_table(b, &b->d_fargs, fargs)) return rc;
   if (int rc = upload_table(b, &b->d_cargs, cargs)) return rc;
@@ -537,7 +586,7 @@ int fgpu_batch_create(fgpu_handle* const* members, int n, fgpu_batch** out) {
   cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, h0->device);
   if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess)
     return fail(FGPU_ECUDA, "stream");
-  b->variant = (h0->variant == 1 || h0->variant >= 4) ? 0 : h0->variant;
+  b->variant = h0->variant >= 6 ? 6 : (h0->variant == 1 || h0->variant >= 4 ? 0 : h0->variant);
   if (b->embedded) b->order = 0;   // no fixed stages: d_args holds the tuner's probes only
   // argument tables: step stages of every member, then the tuner's RHS probes
   std::vector<StageArgs> args((size_t)(b->order + 1) * n);
@@ -608,6 +657,39 @@ int fgpu_batch_create(fgpu_handle* const* members, int n, fgpu_batch** out) {
       cudaMalloc(&b->d_bblocks, sizeof(int4) * bblocks.size()) != cudaSuccess ||
       cudaMallocHost(&b->h_ctls, sizeof(Ctl) * n) != cudaSuccess)
     return fail(FGPU_ENOMEM, "batch tables");
+  // the marching layout's queue: blocks of kStripWarps warps (2D), 32 x 8 tiles times z chunks (3D)
+  {
+    std::vector<int4> queue;
+    auto strips = [](const Grid& g) { return (g.nx + kStripW - 1) / kStripW; };
+    long long warp_rows = 0;
+    for (int i = 0; i < n; ++i) warp_rows += (long long)strips(b->m[i]->g) * b->m[i]->g.ny;
+    b->march_rows = strip_rows(warp_rows);
+    b->march_lim = -1;
+    for (int i = 0; i < n; ++i) {
+      fgpu_handle* h = b->m[i];
+      const Grid& g = h->g;
+      const int l = compiled_limiter(h->cfg.limiter, h->cfg.order == FGPU_CONSTANT, h->cfg.theta);
+      b->march_lim = b->march_lim < 0 || b->march_lim == l ? l : 0;
+      if (b->nd == 2) {
+        const int warps = strips(g) * ((g.ny + b->march_rows - 1) / b->march_rows);
+        for (int w = 0; w < warps; w += kStripWarps) queue.push_back(make_int4(i, w, stage_has_tmap(h) ? 1 : 0, 0));
+      } else {
+        const int tx = (g.nx + kTmaTX - 1) / kTmaTX, ty = (g.ny + kTmaTY - 1) / kTmaTY;
+        const int tz = (g.nz + h->kchunk - 1) / h->kchunk;
+        for (int z = 0; z < tz; ++z)
+          for (int y = 0; y < ty; ++y)
+            for (int x = 0; x < tx; ++x) queue.push_back(make_int4(i | (stage_has_tmap(h) ? 1 << 30 : 0), x, y, z));
+      }
+    }
+    b->march = true;
+    if (int rc = build_march_table(b, args, b->march_args)) return fail(rc, b->err);
+    if (b->march) {
+      if (int rc = upload_table(b, &b->d_mqueue, queue)) return fail(rc, b->err);
+      if (b->nd == 2) (b->euler ? strip2_batch_configure_euler : strip2_batch_configure_iso)(b->prim, b->march_lim);
+      else (b->euler ? march3_batch_configure_euler : march3_batch_configure_iso)(b->prim, b->march_lim);
+      b->nmqueue = (int)queue.size();
+    }
+  }
   cudaMemcpyAsync(b->d_args, args.data(), sizeof(StageArgs) * args.size(), cudaMemcpyHostToDevice, b->stream);
   cudaMemcpyAsync(b->d_bnd, bnd.data(), sizeof(BndArgs) * bnd.size(), cudaMemcpyHostToDevice, b->stream);
   cudaMemcpyAsync(b->d_tiles, tiles.data(), sizeof(int4) * tiles.size(), cudaMemcpyHostToDevice, b->stream);
@@ -627,52 +709,8 @@ int fgpu_batch_create(fgpu_handle* const* members, int n, fgpu_batch** out) {
     b->nfab = (int)fab.size();
     b->nfwcb = (int)fwcb.size();
   }
-  // tensor maps of every stage input for the TMA layout: fixed-step 2D members whose stages
-  // it serves (the same conditions as a lone grid's), the limiter compiled in when shared
-  if (b->nd == 2 && !b->embedded) {
-    std::vector<CUtensorMap> maps(args.size());
-    bool ok = true;
-    int lim = -2;
-    for (size_t q = 0; q < args.size() && ok; ++q) {
-      fgpu_handle* h = b->m[q % n];
-      const StageArgs& A = args[q];
-      ok = tma_eligible(h, A);
-      if (!ok) break;
-      const StateRef& SR = A.rin.base ? A.rin : A.in;
-      const CUtensorMap* mp = stage_tmap(h, SR.base, kTmaTX, kTmaTY);
-      ok = mp != nullptr;
-      if (ok) maps[q] = *mp;
-      const int l = compiled_limiter(A.limiter, A.constant_recon != 0, A.theta);
-      lim = lim == -2 ? l : (lim == l ? lim : 0);
-    }
-    if (ok && !args.empty()) {
-      // blocks of tpb tiles along y (the boxes double-buffered); the 2D stage arguments carry
-      // tpb in kchunk, which the shared-memory tiles of 2D meshes do not read
-      const int tpb = tma_tiles_per_block(b->ntiles, 3);
-      std::vector<int4> cols;
-      for (int i = 0; i < n; ++i) {
-        const Grid& g = b->m[i]->g;
-        const int tx = (g.nx + kTmaTX - 1) / kTmaTX, tyb = ((g.ny + kTmaTY - 1) / kTmaTY + tpb - 1) / tpb;
-        for (int y = 0; y < tyb; ++y)
-          for (int x = 0; x < tx; ++x) cols.push_back(make_int4(i, x, y, 0));
-      }
-      for (auto& A : args) A.kchunk = tpb;
-      b->ntcols = (int)cols.size();
-      // stages whose arguments reduce CFL / CheckData / error maxima for some member
-      b->tma_red.assign(b->order + 1, 0);
-      for (size_t q = 0; q < args.size(); ++q)
-        if (args[q].cfl_mode || args[q].last_stage || args[q].err_low) b->tma_red[q / n] = 1;
-      if (cudaMalloc(&b->d_maps, sizeof(CUtensorMap) * maps.size()) != cudaSuccess ||
-          cudaMemcpy(b->d_maps, maps.data(), sizeof(CUtensorMap) * maps.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-          cudaMalloc(&b->d_tcols, sizeof(int4) * cols.size()) != cudaSuccess ||
-          cudaMemcpy(b->d_tcols, cols.data(), sizeof(int4) * cols.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-          cudaMemcpy(b->d_args, args.data(), sizeof(StageArgs) * args.size(), cudaMemcpyHostToDevice) != cudaSuccess)
-        return fail(FGPU_ENOMEM, "batch tensor maps");
-      b->tma_lim = lim;
-      if (h0->variant >= 6) b->variant = 6;
-    }
-  }
   if (b->embedded) { if (int rc = build_embedded_tables(b)) return fail(rc, b->err); }
+  if (!b->march && b->variant == 6) b->variant = 0;
   *out = b;
   return FGPU_OK;
 }
@@ -682,8 +720,8 @@ void fgpu_batch_destroy(fgpu_batch* b) {
   if (b->stream) cudaStreamSynchronize(b->stream);
   if (b->graph) cudaGraphExecDestroy(b->graph);
   if (b->d_args) cudaFree(b->d_args);
-  if (b->d_maps) cudaFree(b->d_maps);
-  if (b->d_tcols) cudaFree(b->d_tcols);
+  for (void* p : {(void*)b->d_mqueue, (void*)b->march_args.d_maps, (void*)b->march_eargs.d_maps})
+    if (p) cudaFree(p);
   if (b->d_bnd) cudaFree(b->d_bnd);
   if (b->d_tiles) cudaFree(b->d_tiles);
   if (b->d_bblocks) cudaFree(b->d_bblocks);
@@ -774,8 +812,7 @@ int fgpu_batch_autotune(fgpu_batch* b, int reps, int* variant) {
   if (!b) return FGPU_EARG;
   if (reps < 1) reps = 3;
   const StageArgs* probe = b->d_args + (size_t)b->order * b->m.size();
-  std::vector<int> cand = {0, 2, 3};
-  if (b->d_maps) cand.push_back(6);
+  const int cand[3] = {0, 2, 3};
   double best = 1e300;
   int bv = b->variant;
   for (int v : cand) {
@@ -867,24 +904,39 @@ int fgpu_autotune(fgpu_handle* h, int reps, int* variant) {
       A.out = h->buf[2 + m - 1];
       set_fnext(h, A, m, h->dt, nullptr);
     } else if (!h->butcher && !h->adaptive_me && h->order >= 3) {
-      // a middle Shu-Osher stage: scratch state in, scratch state out, the stored state as y0
+      // a middle Shu-Osher stage of the stored state into a scratch state
       A = shu_osher_stage(h, 2);
+      A.in.base = h->buf[0];
+      A.dt_dev = nullptr;   // dt 0: the timed results stay states
       A.ctl = nullptr;
       A.cfl_mode = 0;
     }
+    // formed stage inputs hold the stored state: cells without a state (zeros) would be timed on
+    // the arithmetic's slow paths
+    if (A.rin.base)
+      if (int rc = launch_form(h, plain_state(h->buf[0], false), const_cast<double*>(A.rin.base))) return rc;
+    if (A.fnext_out && !h->first_done) {
+      // the cold state is scratch until FirstStep writes it
+      CUDA_TRY(h, cudaMemcpyAsync(h->buf[1], h->buf[0], sizeof(double) * h->V * h->g.n, cudaMemcpyDeviceToDevice,
+                                  h->stream));
+    }
   } else if (h->fargo && !h->vis && !h->accrete && !h->butcher && !h->adaptive_me && h->order >= 3) {
-    // a middle FARGO Shu-Osher stage with its frame changes (scratch in, scratch out)
+    // a middle FARGO Shu-Osher stage with its frame changes, of the stored state into a scratch state
     A = fargo_stage_args(h, fargo_step_of(h), 2);
+    A.in.base = h->buf[0];
+    A.dt_dev = nullptr;
     A.ctl = nullptr;
     A.cfl_mode = 0;
   }
-  const int cand[8] = {0, 2, 3, 4, 5, 1, 6, 7};
+  // (6 is what 0 launches where the marching kernels serve the stage)
+  const int cand[7] = {0, 2, 3, 4, 5, 1, 7};
   // 3D: the z extent a block marches through (smaller chunks give small grids more blocks);
   // FGPU_KCHUNK fixes it
   std::vector<int> chunks;
   if (h->nd == 3 && !std::getenv("FGPU_KCHUNK")) {
+    chunks.push_back(march_chunk(h->g, 1));
     for (int kc : {4, 8, 16, 32})
-      if (kc <= std::max(4, h->g.nz)) chunks.push_back(kc);
+      if (kc <= std::max(4, h->g.nz) && kc != chunks[0]) chunks.push_back(kc);
   } else {
     chunks.push_back(h->kchunk);
   }
@@ -894,9 +946,8 @@ int fgpu_autotune(fgpu_handle* h, int reps, int* variant) {
   for (int v : cand) {
     // layout 1 lacks these features (Butcher steps gate their stages or form the next stage's state)
     if (v == 1 && (h->fargo || h->accrete || h->vis || h->butcher)) continue;
-    // layouts 6, 7 (TMA-staged planes) serve grids without viscosity or accretion, even nx
-    if (v >= 6 && (h->accrete || h->vis || h->g.nx % 2 != 0)) continue;
-    if (v == 7 && h->nd == 3) continue;   // the 32 x 4 TMA tile is built for 2D meshes
+    // 7: the 2D strips with half the rows per warp
+    if (v == 7 && (h->accrete || h->nd == 3 || strip_rows(strip_warp_rows(h->g)) == 1)) continue;
     // the taller tiles (4, 5) differ from the oracle in the last bit on FARGO transport along x
     // with a user-supplied background velocity; such grids keep the 32 x 8 tiles
     if ((v == 4 || v == 5) && h->fargo && h->fdir == 1) continue;

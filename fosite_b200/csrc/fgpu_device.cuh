@@ -211,6 +211,12 @@ template <int LO, int HI>
 __device__ __forceinline__ bool in_range(double x) {
   return (unsigned)(__double2hiint(x) - ((1023 - LO) << 20)) < (unsigned)((HI + LO) << 20);
 }
+// the IEEE forms for arguments out of range, out of line: the stage kernels' loops stay small
+static __device__ __noinline__ double rcp_ieee(double d) { return 1. / d; }
+static __device__ __noinline__ double sound_speed_ieee(double s, double rho, double floor2) {
+  const double c2 = s / rho;
+  return sqrt(c2 > floor2 ? c2 : floor2);   // (the floor for a NaN, like FP64 max)
+}
 #endif
 
 // ---------------------------------------------------------------- physics
@@ -220,12 +226,14 @@ struct Phys {
   static constexpr int V = EU ? ND + 2 : ND + 1;
 
   // Cons2Prim (physics_euler.f90:3064-3100, physics_eulerisotherm.f90:2831-2856)
+  // (CHECKED = false: a density out of range makes p NaN, which the caller tests for)
+  template <bool CHECKED = true>
   static __device__ __forceinline__ void c2p(const double* c, double* p, const PhysP& P) {
 #ifdef FGPU_EXACT
     double inv_rho = 1. / c[0];
 #else
     double inv_rho = rcp_refined(c[0]);
-    if (!in_range<1000, 1000>(c[0])) inv_rho = 1. / c[0];   // zero, negative, extreme or NaN densities
+    if (CHECKED && !in_range<1000, 1000>(c[0])) inv_rho = rcp_ieee(c[0]);   // zero, negative, extreme or NaN densities
 #endif
     p[0] = c[0];
 #pragma unroll
@@ -253,17 +261,26 @@ struct Phys {
   }
   // GetSoundSpeed (physics_euler.f90:2682-2689): sqrt(MAX(2 TINY, gamma*p/rho)).
   // The product build evaluates sqrt(s/rho) as s*rsqrt(s*rho) with s = gamma*p (within a few
-  // ulp); the range test keeps s*rho and s/rho away from the ends of the double range, where
-  // the reference's form takes over.
+  // ulp).  Wherever s*rho leaves the normal range, or s or rho is not positive, that form gives
+  // a NaN, a negative value or one below the floor sqrt(2 TINY) = 2^-510.5 (cs_good); the
+  // reference's form then takes over.
   static __device__ __forceinline__ double cs_of(const double* p, const PhysP& P) {
 #ifdef FGPU_EXACT
     return sqrt(dmax(P.tiny2, P.gamma * p[V - 1] / p[0]));
 #else
     const double s = P.gamma * p[V - 1];
-    if (in_range<480, 480>(s) && in_range<480, 480>(p[0])) return s * rsqrt_refined(s * p[0]);
-    return sqrt(dmax(P.tiny2, s / p[0]));
+    const double cs = s * rsqrt_refined(s * p[0]);
+    return cs_good(cs) ? cs : sound_speed_ieee(s, p[0], P.tiny2);
 #endif
   }
+#ifndef FGPU_EXACT
+  static __device__ __forceinline__ double cs_fast(const double* p, const PhysP& P) {
+    const double s = P.gamma * p[V - 1];
+    return s * rsqrt_refined(s * p[0]);
+  }
+  // at least 2^-510, finite
+  static __device__ __forceinline__ bool cs_good(double cs) { return in_range<510, 1024>(cs); }
+#endif
 };
 
 // ---------------------------------------------------------------- limiters
@@ -332,6 +349,24 @@ __device__ __forceinline__ double slope(int lim, double theta, double invd, doub
   return invd * limit2(lim, theta, q0 - qm, qp - q0);
 }
 
+// The factor of a slope and of the face offsets that multiply it: the exact build divides the
+// limited difference by the cell width first (as the reference does), the product build multiplies the
+// offset by the inverse width once.
+__device__ __forceinline__ double slope_width(double invd) {
+#ifdef FGPU_EXACT
+  return invd;
+#else
+  return 1.0;
+#endif
+}
+__device__ __forceinline__ double slope_scale(double invd) {
+#ifdef FGPU_EXACT
+  return 1.0;
+#else
+  return invd;
+#endif
+}
+
 // ---------------------------------------------------------------- state access
 template <int V>
 __device__ __forceinline__ void state_at(const StateRef& S, long long n, long long idx, double* u) {
@@ -376,6 +411,81 @@ struct Cells {
     PH::c2p(u, p, P);
   }
 
+  // BC_ABSORBING (boundary_absorbing.f90:114-211): characteristic extrapolation into the first
+  // ghost layer, copied outward.  p1, p2: the primitive variables of the boundary cell and of the
+  // next cell inward along direction d; lo: the face at the low end; ip1, ipR: padded i of the
+  // boundary cell and of the right cell of the pair.
+  static __device__ __noinline__ void absorbing_p(const double* p1, const double* p2, bool lo, int d, int ip1, int ipR,
+                                                  const PhysP& P, const MetricP& M, double* p) {
+    const int delta = lo ? -1 : 1, vn = 1 + d;
+    const double* pL = lo ? p1 : p2;
+    const double* pR = lo ? p2 : p1;
+    double lam[V], xv[V];
+    if (!EU) {
+      // iso: physics_eulerisotherm.f90:1764-2220, elementals :2895-2970
+      double cs1 = M.cs[0 * M.nxp + ip1];
+      double csf = M.cs[(1 + 2 * d) * M.nxp + ipR];          // fcsound(iR, west/south/bottom)
+      double v = p1[vn];
+      lam[0] = v - cs1;
+#pragma unroll
+      for (int t = 1; t < V - 1; ++t) lam[t] = v;
+      lam[V - 1] = v + cs1;
+      double dlnrho = log(pR[0] / pL[0]);
+      double ducs = (pR[vn] - pL[vn]) / csf;
+      xv[0] = dlnrho - ducs;
+      xv[V - 1] = dlnrho + ducs;
+      int t = 1;
+#pragma unroll
+      for (int m = 1; m <= ND; ++m)
+        if (m != vn) { xv[t] = pR[m] - pL[m]; ++t; }
+    } else {
+      // Euler: physics_euler.f90:743-1265, elementals :2799-2890
+      double cs = PH::cs_of(p1, P);
+      double v = p1[vn];
+      double l1 = v - cs, l3 = v + cs;
+      lam[0] = l1;
+#pragma unroll
+      for (int t = 1; t < V - 1; ++t) lam[t] = v;
+      lam[V - 1] = l3;
+      double dlnP = log(pR[V - 1] / pL[V - 1]);
+      double gdu = 2 * P.gamma * (pR[vn] - pL[vn]) / (l3 - l1);
+      xv[0] = dlnP - gdu;
+      xv[1] = dlnP - P.gamma * log(pR[0] / pL[0]);
+      int t = 2;
+#pragma unroll
+      for (int m = 1; m <= ND; ++m)
+        if (m != vn) { xv[t] = pR[m] - pL[m]; ++t; }
+      xv[V - 1] = dlnP + gdu;
+    }
+#pragma unroll
+    for (int l = 0; l < V; ++l)
+      if (lo ? (lam[l] >= 0.0) : (lam[l] <= 0.0)) xv[l] = 0.0;
+    if (!EU) {
+      double csf = M.cs[(1 + 2 * d + (lo ? 0 : 1)) * M.nxp + ip1];
+      p[0] = p1[0] * exp(delta * 0.5 * (xv[V - 1] + xv[0]));
+      p[vn] = p1[vn] + delta * 0.5 * csf * (xv[V - 1] - xv[0]);
+      int t = 1;
+#pragma unroll
+      for (int m = 1; m <= ND; ++m)
+        if (m != vn) { p[m] = p1[m] + delta * xv[t]; ++t; }
+    } else {
+      double dlnP = 0.5 * (xv[V - 1] + xv[0]);
+      double rho2 = p1[0] * exp(delta / P.gamma * (dlnP - xv[1]));
+      double P2 = p1[V - 1] * exp(delta * dlnP);
+      double pa[V];
+      pa[0] = p1[0] + rho2;
+      pa[V - 1] = p1[V - 1] + P2;
+      double cs = PH::cs_of(pa, P);
+      p[0] = rho2;
+      p[V - 1] = P2;
+      p[vn] = p1[vn] + 0.5 * delta * cs / P.gamma * (xv[V - 1] - xv[0]);
+      int t = 2;
+#pragma unroll
+      for (int m = 1; m <= ND; ++m)
+        if (m != vn) { p[m] = p1[m] + delta * xv[t]; ++t; }
+    }
+  }
+
   // Face ghost: exactly one of (i,j,k) outside the interior, in direction d.
   // boundary_periodic.f90:73-116, boundary_reflecting.f90:89-204,
   // boundary_nogradients.f90:75-125, boundary_absorbing.f90:114-211.
@@ -403,82 +513,12 @@ struct Cells {
     } else if (type == BC_NOGRAD) {
       ijk[d] = lo ? 0 : nd - 1;
       interior_p(S, g, P, ijk[0], ijk[1], ijk[2], p);
-    } else {   // BC_ABSORBING: characteristic extrapolation into the first ghost layer, copied outward
+    } else {   // BC_ABSORBING
       int i1 = lo ? 0 : nd - 1, i2 = lo ? 1 : nd - 2;
-      int iL = i1 < i2 ? i1 : i2, iR = i1 < i2 ? i2 : i1;
-      int delta = lo ? -1 : 1;
       double p1[V], p2[V];
       ijk[d] = i1; interior_p(S, g, P, ijk[0], ijk[1], ijk[2], p1);
       ijk[d] = i2; interior_p(S, g, P, ijk[0], ijk[1], ijk[2], p2);
-      const double* pL = (iL == i1) ? p1 : p2;
-      const double* pR = (iR == i1) ? p1 : p2;
-      double lam[V], xv[V];
-      if (!EU) {
-        // iso: physics_eulerisotherm.f90:1764-2220, elementals :2895-2970
-        int ip1 = (d == 0 ? i1 : ijk[0]) + 2;                 // padded i of the boundary cell
-        int ipR = (d == 0 ? iR : ijk[0]) + 2;
-        double cs1 = M.cs[0 * M.nxp + ip1];
-        double csf = M.cs[(1 + 2 * d) * M.nxp + ipR];          // fcsound(iR, west/south/bottom)
-        double v = p1[vn];
-        lam[0] = v - cs1;
-#pragma unroll
-        for (int t = 1; t < V - 1; ++t) lam[t] = v;
-        lam[V - 1] = v + cs1;
-        double dlnrho = log(pR[0] / pL[0]);
-        double ducs = (pR[vn] - pL[vn]) / csf;
-        xv[0] = dlnrho - ducs;
-        xv[V - 1] = dlnrho + ducs;
-        int t = 1;
-#pragma unroll
-        for (int m = 1; m <= ND; ++m)
-          if (m != vn) { xv[t] = pR[m] - pL[m]; ++t; }
-      } else {
-        // Euler: physics_euler.f90:743-1265, elementals :2799-2890
-        double cs = PH::cs_of(p1, P);
-        double v = p1[vn];
-        double l1 = v - cs, l3 = v + cs;
-        lam[0] = l1;
-#pragma unroll
-        for (int t = 1; t < V - 1; ++t) lam[t] = v;
-        lam[V - 1] = l3;
-        double dlnP = log(pR[V - 1] / pL[V - 1]);
-        double gdu = 2 * P.gamma * (pR[vn] - pL[vn]) / (l3 - l1);
-        xv[0] = dlnP - gdu;
-        xv[1] = dlnP - P.gamma * log(pR[0] / pL[0]);
-        int t = 2;
-#pragma unroll
-        for (int m = 1; m <= ND; ++m)
-          if (m != vn) { xv[t] = pR[m] - pL[m]; ++t; }
-        xv[V - 1] = dlnP + gdu;
-      }
-#pragma unroll
-      for (int l = 0; l < V; ++l)
-        if (lo ? (lam[l] >= 0.0) : (lam[l] <= 0.0)) xv[l] = 0.0;
-      if (!EU) {
-        int ip1 = (d == 0 ? i1 : ijk[0]) + 2;
-        double csf = M.cs[(1 + 2 * d + (lo ? 0 : 1)) * M.nxp + ip1];
-        p[0] = p1[0] * exp(delta * 0.5 * (xv[V - 1] + xv[0]));
-        p[vn] = p1[vn] + delta * 0.5 * csf * (xv[V - 1] - xv[0]);
-        int t = 1;
-#pragma unroll
-        for (int m = 1; m <= ND; ++m)
-          if (m != vn) { p[m] = p1[m] + delta * xv[t]; ++t; }
-      } else {
-        double dlnP = 0.5 * (xv[V - 1] + xv[0]);
-        double rho2 = p1[0] * exp(delta / P.gamma * (dlnP - xv[1]));
-        double P2 = p1[V - 1] * exp(delta * dlnP);
-        double pa[V];
-        pa[0] = p1[0] + rho2;
-        pa[V - 1] = p1[V - 1] + P2;
-        double cs = PH::cs_of(pa, P);
-        p[0] = rho2;
-        p[V - 1] = P2;
-        p[vn] = p1[vn] + 0.5 * delta * cs / P.gamma * (xv[V - 1] - xv[0]);
-        int t = 2;
-#pragma unroll
-        for (int m = 1; m <= ND; ++m)
-          if (m != vn) { p[m] = p1[m] + delta * xv[t]; ++t; }
-      }
+      absorbing_p(p1, p2, lo, d, (d == 0 ? i1 : ijk[0]) + 2, (d == 0 ? (lo ? i2 : i1) : ijk[0]) + 2, P, M, p);
     }
   }
 
@@ -579,10 +619,12 @@ struct Cells {
 // 555-686) and CalcFluxes{X,Y,Z}/SetFlux (physics_euler.f90:492-742,
 // physics_eulerisotherm.f90:835-979).  RL: reconstructed variables on the
 // plus face of the left cell, RR: on the minus face of the right cell.
-// DC >= 0: the direction is DC, known at compile time (d_rt is ignored).
-template <int ND, bool EU, bool PRIM, int DC = -1>
+// DC >= 0: the direction is DC, known at compile time (d_rt is ignored).  FAST (product build,
+// ideal gas): straight-line code without the range tests of the conversions and sound speeds;
+// `bad` is set when a sound speed is not good, and the flux then void (kt_flux_try).
+template <int ND, bool EU, bool PRIM, int DC = -1, bool FAST = false>
 __device__ __forceinline__ void kt_flux(int d_rt, const double* RL, const double* RR, double csL_iso, double csR_iso,
-                                        double dA, const PhysP& P, double* F) {
+                                        double dA, const PhysP& P, double* F, bool* bad = nullptr) {
   using PH = Phys<ND, EU>;
   constexpr int V = PH::V;
   const int d = DC >= 0 ? DC : d_rt;
@@ -595,11 +637,26 @@ __device__ __forceinline__ void kt_flux(int d_rt, const double* RL, const double
   } else {
 #pragma unroll
     for (int l = 0; l < V; ++l) { cL[l] = RL[l]; cR[l] = RR[l]; }
-    PH::c2p(cL, pL, P);
-    PH::c2p(cR, pR, P);
+    PH::template c2p<!FAST>(cL, pL, P);
+    PH::template c2p<!FAST>(cR, pR, P);
   }
+#ifdef FGPU_EXACT
   double csL = EU ? PH::cs_of(pL, P) : csL_iso;
   double csR = EU ? PH::cs_of(pR, P) : csR_iso;
+#else
+  double csL, csR;
+  if (!EU) {
+    csL = csL_iso;
+    csR = csR_iso;
+  } else if (FAST) {
+    csL = PH::cs_fast(pL, P);
+    csR = PH::cs_fast(pR, P);
+    *bad = !(PH::cs_good(csL) & PH::cs_good(csR));
+  } else {
+    csL = PH::cs_of(pL, P);
+    csR = PH::cs_of(pR, P);
+  }
+#endif
   const int vn = 1 + d;
   // the normal velocity by selection (d may be a run-time value: no indexed register arrays)
   auto normal = [&](const double* q) {
@@ -645,6 +702,44 @@ __device__ __forceinline__ void kt_flux(int d_rt, const double* RL, const double
   double amap = am * ap;
 #pragma unroll
   for (int l = 0; l < V; ++l) F[l] = fac * (ap * fL[l] - am * fR[l] + amap * (cR[l] - cL[l]));
+}
+
+// The flux with its tests, out of line, for the rare faces whose states the straight-line form
+// does not cover.  Everything goes by value: a reference would keep the callers' states and the
+// kernel's parameters in memory.
+template <int V> struct Face { double v[V]; };
+template <int ND, bool EU, bool PRIM, int D>
+__device__ __noinline__ Face<Phys<ND, EU>::V> kt_flux_checked(Face<Phys<ND, EU>::V> L, Face<Phys<ND, EU>::V> R,
+                                                              double csL_iso, double csR_iso, double dA, PhysP P) {
+  Face<Phys<ND, EU>::V> F;
+  kt_flux<ND, EU, PRIM, D>(D, L.v, R.v, csL_iso, csR_iso, dA, P, F.v);
+  return F;
+}
+// One face flux of direction D as the marching kernels use it: straight-line code (the
+// scheduler can interleave the directions' chains), one rarely taken branch to the checked form.
+template <int ND, bool EU, bool PRIM, int D>
+__device__ __forceinline__ bool kt_flux_try(const double* RL, const double* RR, double csL_iso, double csR_iso,
+                                            double dA, const PhysP& P, double* F) {
+#ifndef FGPU_EXACT
+  if (EU) {
+    bool bad;
+    kt_flux<ND, EU, PRIM, D, true>(D, RL, RR, csL_iso, csR_iso, dA, P, F, &bad);
+    return bad;
+  }
+#endif
+  kt_flux<ND, EU, PRIM, D>(D, RL, RR, csL_iso, csR_iso, dA, P, F);
+  return false;
+}
+template <int ND, bool EU, bool PRIM, int D>
+__device__ __forceinline__ void kt_flux_redo(const double* RL, const double* RR, double csL_iso, double csR_iso,
+                                             double dA, const PhysP& P, double* F) {
+  constexpr int V = Phys<ND, EU>::V;
+  Face<V> L, R;
+#pragma unroll
+  for (int v = 0; v < V; ++v) { L.v[v] = RL[v]; R.v[v] = RR[v]; }
+  const Face<V> f = kt_flux_checked<ND, EU, PRIM, D>(L, R, csL_iso, csR_iso, dA, P);
+#pragma unroll
+  for (int v = 0; v < V; ++v) F[v] = f.v[v];
 }
 
 }  // namespace fgpu

@@ -28,7 +28,7 @@
 #include "fgpu_visc.cuh"
 #include "fgpu_ddmath.h"
 #include "fgpu_bt.cuh"
-#include "fgpu_tma_launch.h"
+#include "fgpu_march_launch.h"
 #include "fgpu_stage_launch.h"
 
 using namespace fgpu;
@@ -168,11 +168,13 @@ struct fgpu_handle {
   bool so_form = false;
   double* d_pform[2] = {nullptr, nullptr};
   double* d_ready = nullptr;    // ... into this array (one state)
-  int variant = 0;              // stage kernel layout: 0 shared-memory tile, 1 warp-shuffle window,
+  int variant = 0;              // stage kernel layout: 0 the default, the marching kernels wherever they
+                                // serve the stage, else the shared-memory base tile; 1 warp-shuffle window,
                                 // 2/3 tile with a register cap for more resident blocks, 4 taller tile,
-                                // 6 tile with TMA-staged planes (fgpu_tma.cuh), 7 its 32 x 4 form (2D)
-  // tensor maps of the stage inputs the TMA layout has read (by base pointer and tile shape)
-  struct TmapEntry { const double* base; int tx, ty; CUtensorMap map; };
+                                // 6 marching kernels (2D fgpu_strip2.cuh, 3D fgpu_march3.cuh), 7 the 2D
+                                // strips with half the rows per warp
+  // tensor maps of the stage inputs the marching layout has read (by base pointer)
+  struct TmapEntry { const double* base; CUtensorMap map; };
   std::vector<TmapEntry> tmaps;
   // instrumentation
   cudaStream_t own_stream = nullptr;
@@ -431,15 +433,15 @@ int upload_metric(fgpu_handle* h) {
 }
 
 // ---------------------------------------------------------------- launchers
-// (the shared-memory stage layouts are launched through fgpu_stage_launch.h, the TMA-staged
-// ones through fgpu_tma_launch.h)
-void configure_stage_kernels(int nd, bool e, bool p) {
+// (the shared-memory stage layouts are launched through fgpu_stage_launch.h, the marching
+// ones through fgpu_march_launch.h)
+void configure_stage_kernels(int nd, bool e, bool p, int lim) {
   if (nd == 2) {
     legacy_stage_configure_2d(e, p);
-    tma_stage_configure_2d(e, p);
+    e ? strip2_configure_euler(p, lim) : strip2_configure_iso(p, lim);
   } else {
     legacy_stage_configure_3d(e, p);
-    tma_stage_configure_3d(e, p);
+    e ? march3_configure_euler(p, lim) : march3_configure_iso(p, lim);
   }
 }
 
@@ -457,16 +459,17 @@ PFN_cuTensorMapEncodeTiled_v12000 tmap_encoder() {
   return fn;
 }
 
-// Tensor map of a state (V fields of n doubles, i fastest) for boxes of (tx+4) x (ty+4) cells
-// of one plane and every variable: dims (nx, ny, [nz,] V); cached per handle by base pointer.
-const CUtensorMap* stage_tmap(fgpu_handle* h, const double* base, int tx, int ty) {
+// Tensor map of a state (V fields of n doubles, i fastest) for the boxes of the marching layouts:
+// dims (nx, ny, [nz,] V), boxes of every variable of one plane of the 3D tile with its halo, or
+// of one row of a 2D strip with its halo; cached per handle by base pointer.
+const CUtensorMap* stage_tmap(fgpu_handle* h, const double* base) {
   for (const auto& e : h->tmaps)
-    if (e.base == base && e.tx == tx && e.ty == ty) return &e.map;
+    if (e.base == base) return &e.map;
   PFN_cuTensorMapEncodeTiled_v12000 enc = tmap_encoder();
   if (!enc) return nullptr;
   const Grid& g = h->g;
   fgpu_handle::TmapEntry e;
-  e.base = base; e.tx = tx; e.ty = ty;
+  e.base = base;
   cuuint64_t dims[4], strides[3];
   cuuint32_t box[4], es[4] = {1, 1, 1, 1};
   int rank;
@@ -474,12 +477,12 @@ const CUtensorMap* stage_tmap(fgpu_handle* h, const double* base, int tx, int ty
     rank = 4;
     dims[0] = g.nx; dims[1] = g.ny; dims[2] = g.nz; dims[3] = h->V;
     strides[0] = 8ull * g.nx; strides[1] = 8ull * g.nx * g.ny; strides[2] = 8ull * g.n;
-    box[0] = tx + 4; box[1] = ty + 4; box[2] = 1; box[3] = h->V;
+    box[0] = kTmaTX + 4; box[1] = kTmaTY + 4; box[2] = 1; box[3] = h->V;
   } else {
     rank = 3;
     dims[0] = g.nx; dims[1] = g.ny; dims[2] = h->V;
     strides[0] = 8ull * g.nx; strides[1] = 8ull * g.n;
-    box[0] = tx + 4; box[1] = ty + 4; box[2] = h->V;
+    box[0] = kStripW + 4; box[1] = 1; box[2] = h->V;
   }
   CUresult r = enc(&e.map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, rank, const_cast<double*>(base), dims, strides, box, es,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -489,34 +492,42 @@ const CUtensorMap* stage_tmap(fgpu_handle* h, const double* base, int tx, int ty
   return &h->tmaps.back().map;
 }
 
-// The TMA layout serves stages whose input is a plain or formed state (no k-sums at the stencil
-// points) without viscous source or accretion rows, on meshes whose x extent is even (16-byte
-// strides of the tensor map); FARGO frame changes on 2D meshes.
+// The marching layouts serve stages whose input is a plain or formed state (no k-sums at the
+// stencil points) without accretion rows or interface-flux output; FARGO frame changes on 2D
+// meshes, where they apply to the staged points of a plain input.
 bool tma_eligible(const fgpu_handle* h, const StageArgs& A) {
   const StateRef& S = A.rin.base ? A.rin : A.in;
   const bool frames = h->fargo || A.w_sub || S.pre.n || A.in.pre.n || A.yn_chain.n || A.y0_chain.n || A.err_chain.n;
-  return h->g.nx % 2 == 0 && (!frames || h->nd == 2) && !h->vis && !A.visc && !A.brow && !A.flux_out && S.nk == 0 &&
-         (S.pre.n == 0 || &S == &A.in) && tmap_encoder() != nullptr;
+  return (!frames || h->nd == 2) && !A.brow && !A.flux_out && S.nk == 0 && (S.pre.n == 0 || &S == &A.in);
 }
+// the tensor map of a stage input, or an empty one where rows have no 16-byte stride (odd x
+// extent: the kernels then copy by element)
+bool stage_has_tmap(const fgpu_handle* h) { return h->g.nx % 2 == 0 && tmap_encoder() != nullptr; }
 
 template <int ND, bool EU, bool PRIM>
 int launch_stage_t(fgpu_handle* h, StageArgs& A) {
   A.kchunk = h->kchunk;
   const Grid& g = h->g;
-  if ((h->variant == 6 || (h->variant == 7 && ND == 2)) && tma_eligible(h, A)) {
+  if ((h->variant == 0 || h->variant >= 6) && tma_eligible(h, A)) {
     const StateRef& SR = A.rin.base ? A.rin : A.in;
-    const int ty = h->variant == 7 ? 4 : kTmaTY;
-    const CUtensorMap* map = stage_tmap(h, SR.base, kTmaTX, ty);
+    const int lim = compiled_limiter(A.limiter, A.constant_recon != 0, A.theta);
+    const bool tma = stage_has_tmap(h);
+    static const CUtensorMap no_map = {};
+    const CUtensorMap* map = tma ? stage_tmap(h, SR.base) : &no_map;
     if (!map) return set_err(h, FGPU_ECUDA, "cuTensorMapEncodeTiled failed for a stage input");
-    const bool crec = A.constant_recon != 0;
-    if (ND == 3) CUDA_TRY(h, tma_stage_launch_3d(EU, PRIM, A.limiter, crec, g, h->kchunk, h->stream, A, *map));
-    else CUDA_TRY(h, tma_stage_launch_2d(EU, PRIM, A.limiter, crec, ty, g, h->stream, A, *map));
+    if (ND == 3) {
+      CUDA_TRY(h, (EU ? march3_launch_euler : march3_launch_iso)(PRIM, lim, h->kchunk, h->stream, A, *map, tma));
+    } else {
+      int rows = strip_rows(strip_warp_rows(g));
+      if (h->variant == 7) rows = std::max(1, rows / 2);
+      CUDA_TRY(h, (EU ? strip2_launch_euler : strip2_launch_iso)(PRIM, lim, rows, h->stream, A, *map, tma));
+    }
     return FGPU_OK;
   }
   // the warp-shuffle layout implements neither FARGO frame changes, the accretion rows, the
   // viscous source, the device-clock gates, the next Butcher stage's state formation nor the
   // CheckData-only epilogue
-  // (a variant-6 launch that the TMA layout does not serve runs on the base tile)
+  // (a launch that the marching layout does not serve runs on the base tile)
   const int variant =
       (h->variant == 1 && (h->fargo || h->accrete || h->vis || A.gate || A.fnext_out || A.cfl_mode == 3 ||
                            A.flux_out || A.out_prim))
@@ -1698,13 +1709,16 @@ int fgpu_create(const fgpu_config* cfg, int device, fgpu_handle** out) {
     if (h->fargo && h->butcher) h->materialize = false;
     h->fuse_form = h->fuse_form && h->materialize;
   }
-  if (!rc) configure_stage_kernels(h->nd, h->euler, h->prim);
+  if (!rc)
+    configure_stage_kernels(h->nd, h->euler, h->prim,
+                            compiled_limiter(cfg->limiter, cfg->order == FGPU_CONSTANT, cfg->theta));
   if (!rc && h->vis) configure_visc(h->nd, h->euler);
   if (!rc) rc = build_metric(h);
   if (!rc) {
     h->g.nx = cfg->inum; h->g.ny = cfg->jnum; h->g.nz = h->nd == 3 ? cfg->knum : 1;
     h->g.n = (long long)h->g.nx * h->g.ny * h->g.nz;
     for (int f = 0; f < 6; ++f) h->g.bc[f] = cfg->bc[f];
+    if (h->nd == 3 && !std::getenv("FGPU_KCHUNK")) h->kchunk = march_chunk(h->g, 1);
     h->g.fdir = h->fdir;
     h->ph.gamma = cfg->gamma; h->ph.gm1 = cfg->gamma - 1.; h->ph.pmin = cfg->pmin; h->ph.rhomin = cfg->rhomin;
     h->ph.tiny2 = 2.0 * DBL_MIN;

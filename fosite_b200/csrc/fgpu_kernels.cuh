@@ -155,20 +155,53 @@ __device__ __forceinline__ void prefetch_l2(const double* p) {
   asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }
 
+// a stage that stage_cell_epilogue serves with SRC = false
+inline bool plain_stage(const StageArgs& A) {
+  return !A.mt.curv && !A.has_accel && !A.visc && !A.w_sub && !A.in.pre.n && !A.yn_chain.n && !A.y0_chain.n &&
+         !A.err_chain.n;
+}
+
+// The arrays that stage_cell_epilogue reads, for their prefetch into L2: the next Butcher
+// stage's base and earlier k, then the stage input's base and k (the last stage's high/low-order
+// sums, or cvar read by the sources), y0, err_low.  None when rows do not start on 16-byte
+// boundaries (aligned = false), which the bulk prefetch needs.
+template <bool EU, bool PRIM>
+struct EpilogueStreams {
+  int nf, nin, n;
+  __device__ __forceinline__ EpilogueStreams(const StageArgs& A, bool aligned) {
+    const bool roundtrip = EU && A.in.roundtrip;
+    const bool in_needed = A.last_stage || A.w_sub || A.yn_chain.n ||
+                           (PRIM && !roundtrip && (A.mt.curv || A.has_accel || A.out_base || A.out_mode == OUT_SSPRK)) ||
+                           (!PRIM && roundtrip);
+    nf = A.fnext_out ? A.fnext.nk : 0;
+    nin = !in_needed ? 0 : (A.last_stage ? A.nstage : A.in.nk + 1);
+    n = !aligned ? 0 : nf + nin + (A.out_mode == OUT_SSPRK ? 1 : 0) + (A.err_low ? 1 : 0);
+  }
+  __device__ __forceinline__ const double* ptr(const StageArgs& A, int q) const {
+    if (q < nf) return q == 0 ? A.fnext.base : A.fnext.K[q - 1];
+    q -= nf;
+    if (q < nin) return q == 0 ? A.in.base : A.in.K[q - 1];
+    q -= nin;
+    if (A.out_mode == OUT_SSPRK && q-- == 0) return A.y0;
+    return A.err_low;
+  }
+};
+
 // The per-cell part of one right-hand side after the flux divergence: the centre state as
 // ComputeRHS sees it, geometric and external sources (timedisc_base.f90:1263-1267), and the
 // stage's consumer (k_m and the next Butcher stage's state, the Shu-Osher update, the embedded
 // solutions and error norm, CheckData and CFL partial maxima).  R0: the cell's reconstruction
 // variables; rhs: (divX + divY) + divZ on entry, the full right-hand side after the sources.
-// Shared by the stage kernels of every tile layout.
-template <int ND, bool EU, bool PRIM, bool KSEQ = false>
+// Shared by the stage kernels of every tile layout.  SRC = false: a stage without geometric,
+// point-mass or viscous sources and without frame changes (plain_stage), whose code is left out.
+template <int ND, bool EU, bool PRIM, bool KSEQ = false, bool SRC = true>
 __device__ __forceinline__ void stage_cell_epilogue(const StageArgs& A, const int i, const int j, const int k,
                                                     const double* R0, double* rhs, const double dt, double* cflv,
                                                     double& errv, int& flags) {
   using PH = Phys<ND, EU>;
   using CE = Cells<ND, EU>;
   constexpr int V = PH::V;
-  constexpr bool FG = ND == 2;   // FARGO transforms are compiled for 2D meshes only
+  constexpr bool FG = SRC && ND == 2;   // FARGO transforms are compiled for 2D meshes only
   const Grid& g = A.g;
   const PhysP& P = A.ph;
   const MetricP& M = A.mt;
@@ -189,7 +222,7 @@ __device__ __forceinline__ void stage_cell_epilogue(const StageArgs& A, const in
     for (int v = 0; v < V; ++v) pc[v] = R0[v];
     // the sources read cvar itself (the stage state), which Prim2Cons(pvar) only
     // reproduces to rounding; after the CHECK_PMIN round trip cvar is Prim2Cons(pvar)
-    if (!roundtrip && (M.curv || A.has_accel || A.out_base)) state_at<V>(A.in, g.n, idx, cc);
+    if (!roundtrip && ((SRC && (M.curv || A.has_accel)) || A.out_base)) state_at<V>(A.in, g.n, idx, cc);
     else PH::p2c(pc, cc, P);
   } else {
 #pragma unroll
@@ -222,27 +255,27 @@ __device__ __forceinline__ void stage_cell_epilogue(const StageArgs& A, const in
     // one (isothermal physics_eulerisotherm.f90:1462-1518; Euler physics_euler.f90:2267-2355
     // adds the energy term -vx*(tmp + GetGeometricalSourceX(vz = P = mz = 0)))
     const double vx = pc[1], vy = pc[2];
-    const double cxyx = M.cxyx[ip], cyxy = M.cyxy[ip], czxz = M.czxz[ip], czyz = M.czyz[ip];
+    const double cxyx = __ldg(M.cxyx + ip), cyxy = __ldg(M.cyxy + ip), czxz = __ldg(M.czxz + ip), czyz = __ldg(M.czyz + ip);
     double geo1 = 0.0;
     if (M.curv) {
-      const double Pp = EU ? pc[V - 1] : pc[0] * (M.cs[ip] * M.cs[ip]);
+      const double Pp = EU ? pc[V - 1] : pc[0] * (__ldg(M.cs + ip) * __ldg(M.cs + ip));
       geo1 = cc[2] * (cyxy * vy - cxyx * vx) + (cyxy + czxz) * Pp;
       rhs[2] = rhs[2] - (cc[1] * (cxyx * vx - cyxy * vy) + (cxyx + czyz) * Pp);
     }
     const int jp = j + 2;
-    const double tmp = cc[2] * 0.5 * (A.w_sub[jp + 1] - A.w_sub[jp - 1]) / M.dly[ip];
+    const double tmp = cc[2] * 0.5 * (__ldg(A.w_sub + jp + 1) - __ldg(A.w_sub + jp - 1)) / __ldg(M.dly + ip);
     geo1 = geo1 - tmp;
     rhs[1] = rhs[1] - geo1;
     if (EU) {
-      const double cxzx = M.cxzx[ip];
+      const double cxzx = __ldg(M.cxzx + ip);
       const double gx = cc[2] * (cyxy * vy - cxyx * vx) + 0.0 * (czxz * 0.0 - cxzx * vx) + (cyxy + czxz) * 0.0;
       const double geoE = 0.0 - vx * (tmp + gx);
       rhs[V - 1] = rhs[V - 1] - geoE;
     }
-  } else if (M.curv && ND == 2 && fsrc) {
-    double Pp = EU ? pc[V - 1] : pc[0] * (M.cs[ip] * M.cs[ip]);
+  } else if (FG && M.curv && fsrc) {
+    double Pp = EU ? pc[V - 1] : pc[0] * (__ldg(M.cs + ip) * __ldg(M.cs + ip));
     double vx = pc[1], vy = pc[2];
-    double cxyx = M.cxyx[ip], cyxy = M.cyxy[ip], czxz = M.czxz[ip], czyz = M.czyz[ip];
+    double cxyx = __ldg(M.cxyx + ip), cyxy = __ldg(M.cyxy + ip), czxz = __ldg(M.czxz + ip), czyz = __ldg(M.czyz + ip);
     rhs[1] = rhs[1] - (cc[2] * (cyxy * vy - cxyx * vx) + (cyxy + czxz) * Pp);
     geo2 = cc[1] * (cxyx * vx - cyxy * vy) + (cxyx + czyz) * Pp;
   }
@@ -250,27 +283,27 @@ __device__ __forceinline__ void stage_cell_epilogue(const StageArgs& A, const in
     // AddFargoSourcesY into the geometric source (isothermal
     // physics_eulerisotherm.f90:1531-1586; Euler physics_euler.f90:2368-2455 adds the
     // energy term -vy*(tmp + GetGeometricalSourceY(vz = P = mz = 0)))
-    const double tmp = cc[1] * 0.5 * (A.w_sub[ip + 1] - A.w_sub[ip - 1]) / M.dlx[ip];
+    const double tmp = cc[1] * 0.5 * (__ldg(A.w_sub + ip + 1) - __ldg(A.w_sub + ip - 1)) / __ldg(M.dlx + ip);
     geo2 = geo2 - tmp;
     rhs[2] = rhs[2] - geo2;
     if (EU) {
       const double vx = pc[1], vy = pc[2];
-      const double cxyx = M.cxyx[ip], cyxy = M.cyxy[ip], cyzy = M.cyzy[ip], czyz = M.czyz[ip];
+      const double cxyx = __ldg(M.cxyx + ip), cyxy = __ldg(M.cyxy + ip), cyzy = __ldg(M.cyzy + ip), czyz = __ldg(M.czyz + ip);
       const double gy = 0.0 * (czyz * 0.0 - cyzy * vy) + cc[1] * (cxyx * vx - cyxy * vy) + (cxyx + czyz) * 0.0;
       const double geoE = 0.0 - vy * (tmp + gy);
       rhs[V - 1] = rhs[V - 1] - geoE;
     }
-  } else if (!fsrc && M.curv) {
-    double Pp = EU ? pc[V - 1] : pc[0] * (M.cs[ip] * M.cs[ip]);
+  } else if (SRC && !fsrc && M.curv) {
+    double Pp = EU ? pc[V - 1] : pc[0] * (__ldg(M.cs + ip) * __ldg(M.cs + ip));
     double vx = pc[1], vy = pc[2];
-    double cxyx = M.cxyx[ip], cyxy = M.cyxy[ip], czxz = M.czxz[ip], czyz = M.czyz[ip];
+    double cxyx = __ldg(M.cxyx + ip), cyxy = __ldg(M.cyxy + ip), czxz = __ldg(M.czxz + ip), czyz = __ldg(M.czyz + ip);
     if (ND == 2) {
       double mx = cc[1], my = cc[2];
       rhs[1] = rhs[1] - (my * (cyxy * vy - cxyx * vx) + (cyxy + czxz) * Pp);
       rhs[2] = rhs[2] - (mx * (cxyx * vx - cyxy * vy) + (cxyx + czyz) * Pp);
     } else {
       double vz = pc[3], mx = cc[1], my = cc[2], mz = cc[3];
-      double cxzx = M.cxzx[ip], cyzy = M.cyzy[ip];
+      double cxzx = __ldg(M.cxzx + ip), cyzy = __ldg(M.cyzy + ip);
       rhs[1] = rhs[1] - (my * (cyxy * vy - cxyx * vx) + mz * (czxz * vz - cxzx * vx) + (cyxy + czxz) * Pp);
       rhs[2] = rhs[2] - (mz * (czyz * vz - cyzy * vy) + mx * (cxyx * vx - cyxy * vy) + (cxyx + czyz) * Pp);
       rhs[3] = rhs[3] - (mx * (cxzx * vx - czxz * vz) + my * (cyzy * vy - czyz * vz) + (cxzx + cyzy) * Pp);
@@ -279,10 +312,10 @@ __device__ __forceinline__ void stage_cell_epilogue(const StageArgs& A, const in
   // external sources (sources_generic.f90:220-261): point-mass gravity (gravity_pointmass.f90:
   // 263-282, physics ExternalSources) first in the list, then the viscous source of this
   // stage state (precomputed by visc_kernel); rhs = ... - (gravity + viscosity)
-  if (A.has_accel || A.visc) {
+  if (SRC && (A.has_accel || A.visc)) {
     double sm[ND] = {}, se = 0.0;
     if (A.has_accel) {
-      const double ax = M.accel[ip], ay = M.accel[M.nxp + ip];
+      const double ax = __ldg(M.accel + ip), ay = __ldg(M.accel + M.nxp + ip);
       sm[0] = cc[0] * ax;
       sm[1] = cc[0] * ay;
       if (EU) se = cc[1] * ax + cc[2] * ay;
@@ -317,13 +350,14 @@ __device__ __forceinline__ void stage_cell_epilogue(const StageArgs& A, const in
       // the earlier stages' k: unrolled to the tableau limit, so that all loads issue together,
       // or (KSEQ: kernels short of registers, whose streams the L2 prefetch has brought in) one
       // k at a time
+      const double dtd = S.dt_dev ? *S.dt_dev : 1.0;
       auto kterm = [&](int q) {
-        const double a = S.dt_dev ? S.coef[q] * *S.dt_dev : S.coef[q];
+        const double a = S.coef[q] * dtd;
 #pragma unroll
         for (int v = 0; v < V; ++v) u[v] = u[v] - a * __ldg(S.K[q] + (long long)v * g.n + idx);
       };
       if (KSEQ) {
-#pragma unroll 1
+#pragma unroll 2
         for (int q = 0; q + 1 < S.nk; ++q) kterm(q);
       } else {
 #pragma unroll
@@ -331,7 +365,7 @@ __device__ __forceinline__ void stage_cell_epilogue(const StageArgs& A, const in
           if (q + 1 < S.nk) kterm(q);
       }
       {
-        const double a = S.dt_dev ? S.coef[S.nk - 1] * *S.dt_dev : S.coef[S.nk - 1];
+        const double a = S.coef[S.nk - 1] * dtd;
 #pragma unroll
         for (int v = 0; v < V; ++v) u[v] = u[v] - a * rhs[v];
       }
@@ -402,7 +436,7 @@ __device__ __forceinline__ void stage_cell_epilogue(const StageArgs& A, const in
       double p[V], c[V];
       PH::c2p(y, p, P);
       if (EU && A.cfl_roundtrip) p[V - 1] = dmax(p[V - 1], P.pmin);
-      double cs = EU ? PH::cs_of(p, P) : M.cs[ip];
+      double cs = EU ? PH::cs_of(p, P) : __ldg(M.cs + ip);
       double v3[4];
       CE::cfl_cell(p, cs, M, ip, v3);
 #pragma unroll
@@ -424,13 +458,13 @@ __device__ __forceinline__ void stage_cell_epilogue(const StageArgs& A, const in
       double o[V];
 #pragma unroll
       for (int v = 0; v < V; ++v) o[v] = cc[v];
-      frame_change<V>(o, -1.0, A.w_sub[fargo_ix(g, i, j)], g.fdir);
+      frame_change<V>(o, -1.0, __ldg(A.w_sub + fargo_ix(g, i, j)), g.fdir);
 #pragma unroll
       for (int v = 0; v < V; ++v) A.out_base[(long long)v * g.n + idx] = o[v];
     }
   }
   if (A.cfl_mode >= 2) {
-    double cs = EU ? PH::cs_of(pc, P) : M.cs[ip];
+    double cs = EU ? PH::cs_of(pc, P) : __ldg(M.cs + ip);
     if (A.cfl_mode == 2) {
       double v3[4];
       CE::cfl_cell(pc, cs, M, ip, v3);
@@ -448,13 +482,13 @@ __device__ __forceinline__ void stage_cell_epilogue(const StageArgs& A, const in
     // timedisc_base.f90:1012-1053); base and the earlier k unrolled to the tableau limit
     // so that their loads issue together, this stage's k from the registers.  On the
     // device clock (in.dt_dev) bh_dt/bl_dt hold the weights, multiplied by *dt_dev here.
-    const double* dtd = A.in.dt_dev;
+    const double dtd = A.in.dt_dev ? *A.in.dt_dev : 1.0;   // (the product with 1 is exact)
     double hi[V], lo[V];
 #pragma unroll
     for (int v = 0; v < V; ++v) hi[v] = lo[v] = __ldg(A.in.base + (long long)v * g.n + idx);
     auto kterm = [&](int q) {
-      const double bh = dtd ? A.bh_dt[q] * *dtd : A.bh_dt[q];
-      const double bl = dtd ? A.bl_dt[q] * *dtd : A.bl_dt[q];
+      const double bh = A.bh_dt[q] * dtd;
+      const double bl = A.bl_dt[q] * dtd;
 #pragma unroll
       for (int v = 0; v < V; ++v) {
         const double kq = __ldg(A.in.K[q] + (long long)v * g.n + idx);
@@ -472,8 +506,8 @@ __device__ __forceinline__ void stage_cell_epilogue(const StageArgs& A, const in
     }
     {
       const int q = A.nstage - 1;
-      const double bh = dtd ? A.bh_dt[q] * *dtd : A.bh_dt[q];
-      const double bl = dtd ? A.bl_dt[q] * *dtd : A.bl_dt[q];
+      const double bh = A.bh_dt[q] * dtd;
+      const double bl = A.bl_dt[q] * dtd;
 #pragma unroll
       for (int v = 0; v < V; ++v) {
         lo[v] = lo[v] - bl * rhs[v];
