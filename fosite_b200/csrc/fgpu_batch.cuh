@@ -408,7 +408,7 @@ int enqueue_batch_slot(fgpu_batch* b) {
     }
     BCUDA_TRY(b, cudaGetLastError());
   }
-  bt_decide_batch_kernel<<<mb, 128, 0, b->stream>>>(b->d_ctlp, b->d_btp, n);
+  bt_decide_batch_kernel<<<(2 * n + 127) / 128, 128, 0, b->stream>>>(b->d_ctlp, b->d_btp, n);
   BCUDA_TRY(b, cudaGetLastError());
   if (int rc = launch_batched_stage(b, b->d_eargs + (size_t)(M - 1) * n, b->variant)) return rc;
   if (int rc = launch_batched_stage(b, b->d_eargs + (size_t)M * n, b->variant)) return rc;

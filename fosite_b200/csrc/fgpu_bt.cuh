@@ -49,13 +49,29 @@ __device__ void bt_begin_body(Ctl* c) {
 }
 __global__ void bt_begin_kernel(Ctl* c) { bt_begin_body(c); }
 
-// timedisc_base.f90:759-814 AdjustTimestep with correctly rounded exp/log
-__device__ double bt_adjust(Ctl* c, const BtParams& P, double maxerr, double dtold_) {
+// timedisc_base.f90:759-814 AdjustTimestep with correctly rounded exp/log.  The two factors of
+// the new step, exp(-log(maxerr)/order) and exp(-beta log(maxerrold/maxerr)), are independent
+// serial chains: a pair of lanes evaluates one each (every lane of the warp calls this).
+struct BtFactors { double err, pi; };
+__device__ __forceinline__ BtFactors bt_factors(const Ctl* c, const BtParams& P) {
+  const bool second = threadIdx.x & 1;
+  double y = 0.0;
+  if ((c->act & ACT_ATTEMPT) && !(c->stop | c->brk) && P.tol_rel < 1.0) {
+    const double maxerr = __longlong_as_double((long long)c->err);
+    if (second ? c->maxerrold > 0. : maxerr > 0.) {
+      const double l = ddm::log_cr(second ? c->maxerrold / maxerr : maxerr);
+      y = ddm::exp_cr(second ? -P.beta * l : -l / P.order);
+    }
+  }
+  const double o = __shfl_xor_sync(0xffffffffu, y, 1);
+  return second ? BtFactors{o, y} : BtFactors{y, o};
+}
+__device__ double bt_adjust(Ctl* c, const BtParams& P, const BtFactors& f, double maxerr, double dtold_) {
   double dtnew, dttmp;
   if (P.tol_rel >= 1.0) return DBL_MAX;
-  if (maxerr > 0.) dttmp = 0.9 * dtold_ * ddm::exp_cr(-ddm::log_cr(maxerr) / P.order);
+  if (maxerr > 0.) dttmp = 0.9 * dtold_ * f.err;
   else dttmp = 4. * dtold_;
-  if (c->maxerrold > 0.) dtnew = dttmp * ddm::exp_cr(-P.beta * ddm::log_cr(c->maxerrold / maxerr));
+  if (c->maxerrold > 0.) dtnew = dttmp * f.pi;
   else dtnew = dttmp;
   if (maxerr < 1.0) {
     const double cap = 4. * dtold_;
@@ -73,12 +89,12 @@ __device__ double bt_adjust(Ctl* c, const BtParams& P, double maxerr, double dto
 // The body of IntegrationStep's loop after SolveODE (timedisc_base.f90:684-710): break on a
 // NaN/Inf error, RejectSolution or AcceptSolution (timedisc_base.f90:911-1009), the dtlimit
 // test, the loop condition, and the loop's closing (timedisc_base.f90:712-720).
-__device__ void bt_decide_body(Ctl* c, const BtParams& P) {
+__device__ void bt_decide_body(Ctl* c, const BtParams& P, const BtFactors& f) {
   if (!(c->act & ACT_ATTEMPT) || (c->stop | c->brk)) { c->act = 0; return; }
   const double e = __longlong_as_double((long long)c->err);
   c->err = 0ULL;
   c->last_err = e;
-  const double d = bt_adjust(c, P, e, c->dtold_att);
+  const double d = bt_adjust(c, P, f, e, c->dtold_att);
   int act = 0;
   c->rhs_done = 0;
   if (e != e) c->brk = 1;
@@ -107,7 +123,11 @@ __device__ void bt_decide_body(Ctl* c, const BtParams& P) {
   }
   c->act = act;
 }
-__global__ void bt_decide_kernel(Ctl* c, BtParams P) { bt_decide_body(c, P); }
+// one warp; lane 0 decides
+__global__ void bt_decide_kernel(Ctl* c, BtParams P) {
+  const BtFactors f = bt_factors(c, P);
+  if (threadIdx.x == 0) bt_decide_body(c, P, f);
+}
 
 // CheckData of AcceptSolution's ComputeRHS inside the step (timedisc_base.f90:926-931): a
 // failure breaks IntegrationStep's loop; the step then ends without its closing (time, dt and
@@ -173,9 +193,11 @@ __global__ void bt_begin_batch_kernel(Ctl* const* ctls, int n) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) bt_begin_body(ctls[i]);
 }
+// two lanes per member (bt_factors), the first decides
 __global__ void bt_decide_batch_kernel(Ctl* const* ctls, const BtParams* P, int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) bt_decide_body(ctls[i], P[i]);
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) / 2, m = i < n ? i : n - 1;
+  const BtFactors f = bt_factors(ctls[m], P[m]);
+  if (i < n && !(threadIdx.x & 1)) bt_decide_body(ctls[i], P[i], f);
 }
 __global__ void bt_finish_batch_kernel(Ctl* const* ctls, int n, int nd) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;

@@ -2215,7 +2215,7 @@ static int enqueue_bt_slot(fgpu_handle* h) {
   bp.order = T.order;
   bp.beta = h->beta;
   bp.tol_rel = h->tol_rel;
-  if (int rc = one([&] { bt_decide_kernel<<<1, 1, 0, h->stream>>>(c, bp); })) return rc;
+  if (int rc = one([&] { bt_decide_kernel<<<1, 32, 0, h->stream>>>(c, bp); })) return rc;
   {   // RejectSolution: the RHS of cold (CHECK_NOTHING); with FARGO it frames cvar
     StageArgs A = base_args(h);
     A.out_mode = OUT_RHS;
