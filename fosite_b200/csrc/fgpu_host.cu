@@ -30,6 +30,7 @@
 #include "fgpu_bt.cuh"
 #include "fgpu_march_launch.h"
 #include "fgpu_stage_launch.h"
+#include "fgpu_transfer.h"
 
 using namespace fgpu;
 
@@ -1684,6 +1685,7 @@ int fgpu_create(const fgpu_config* cfg, int device, fgpu_handle** out) {
   if (!cfg || !out) return set_err(nullptr, FGPU_EARG, "null argument");
   *out = nullptr;
   fgpu_handle* h = new fgpu_handle();
+  Transfer::shared().attach();
   std::memset(&h->stats, 0, sizeof(h->stats));
   h->cfg = *cfg;
   int rc = validate(h);
@@ -1828,6 +1830,7 @@ void fgpu_destroy(fgpu_handle* h) {
   if (h->h_ctl) cudaFreeHost(h->h_ctl);
   if (h->own_stream) h->stream = h->own_stream;
   if (h->stream) cudaStreamDestroy(h->stream);
+  Transfer::shared().detach();
   delete h;
 }
 
@@ -1917,7 +1920,8 @@ int fgpu_upload_state(fgpu_handle* h, int which, const double* data, int64_t n) 
   if (which != FGPU_CVAR && which != FGPU_PVAR) return set_err(h, FGPU_EARG, "upload CVAR or PVAR");
   long long nc = fgpu_cell_count(h);
   if (!h->d_pad) CUDA_TRY(h, cudaMalloc(&h->d_pad, sizeof(double) * 2 * nc * h->V));
-  CUDA_TRY(h, cudaMemcpyAsync(h->d_pad, data, sizeof(double) * nc * h->V, cudaMemcpyHostToDevice, h->stream));
+  CUDA_TRY(h, Transfer::shared().copy(const_cast<double*>(data), h->d_pad, sizeof(double) * nc * h->V, false, h->device,
+                                      h->stream));
   long long blocks = std::min<long long>((h->g.n + 255) / 256, 148 * 16);
   int prim = which == FGPU_PVAR;
   h->stats.launches += 1;
@@ -1992,9 +1996,8 @@ int fgpu_download(fgpu_handle* h, int which, double* out, int64_t n) {
   B.npad = nc;
   if (int rc = launch_misc(h, 2, B)) return rc;
   if (int rc = launch_misc(h, 0, B)) return rc;
-  CUDA_TRY(h, cudaMemcpyAsync(out, which == FGPU_PVAR ? B.out_p : B.out_c, sizeof(double) * nc * h->V,
-                              cudaMemcpyDeviceToHost, h->stream));
-  CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+  CUDA_TRY(h, Transfer::shared().copy(out, which == FGPU_PVAR ? B.out_p : B.out_c, sizeof(double) * nc * h->V, true,
+                                      h->device, h->stream));
   return FGPU_OK;
 }
 

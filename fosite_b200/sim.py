@@ -149,7 +149,7 @@ class Simulation:
 
     def get(self, which):
         n = self.ncells if which == abi.BCCSOUND else self.ncells * self.vnum
-        out = np.zeros(n)
+        out = np.empty(n)
         self._check(self.L.fgpu_download(self.h, which, _ptr(out), out.size))
         if which == abi.BCCSOUND:
             return out.reshape(self.shape)
