@@ -166,8 +166,6 @@ __device__ __forceinline__ bool gated_out(const Ctl* c, int gate) {
 
 enum { BC_NOGRAD = 0x01, BC_PERIODIC = 0x02, BC_REFLECTING = 0x03, BC_AXIS = 0x04, BC_ABSORBING = 0x0D };
 enum { LIM_MINMOD = 1, LIM_MC = 2, LIM_SWEBY = 3, LIM_SUPERBEE = 4, LIM_OSPRE = 5, LIM_VANLEER = 7, LIM_NOLIMIT = 8 };
-// kernel-internal code: MC with theta = 1 (the products theta*difference are exact and skipped)
-enum { LIM_MC1 = 102 };
 
 __device__ __forceinline__ double fsign1(double b) { return signbit(b) ? -1.0 : 1.0; }
 __device__ __forceinline__ double fsign(double a, double b) { return signbit(b) ? -fabs(a) : fabs(a); }
@@ -330,9 +328,6 @@ __device__ __forceinline__ double limit2(int lim, double theta, double a1, doubl
 }
 // slope of q0 with neighbours qm, qp (MONOCENT uses minmod3 of three differences)
 __device__ __forceinline__ double slope(int lim, double theta, double invd, double qm, double q0, double qp) {
-  // MC with theta = 1 is minmod: the central difference is the mean of the one-sided ones, and
-  // rounding is monotonic, so (qp - qm)/2 is never the smallest of the three in magnitude
-  if (lim == LIM_MC1) return invd * limit2(LIM_MINMOD, theta, q0 - qm, qp - q0);
   if (lim == LIM_MC) {
     double a1 = theta * (q0 - qm), a2 = theta * (qp - q0);
     double a3 = 0.5 * (qp - qm);

@@ -26,7 +26,7 @@ template <template <int, bool, bool> class Fam, bool PLAIN, class... T>
 void launch_family(int lim, bool red, bool plain, T... a) {
   switch (lim) {
     case LIM_MINMOD: launch_red<Fam, PLAIN, LIM_MINMOD>(red, plain, a...); break;
-    case LIM_MC1: launch_red<Fam, PLAIN, LIM_MC1>(red, plain, a...); break;
+    case LIM_MC: launch_red<Fam, PLAIN, LIM_MC>(red, plain, a...); break;
     case LIM_VANLEER: launch_red<Fam, PLAIN, LIM_VANLEER>(red, plain, a...); break;
     default: launch_red<Fam, PLAIN, 0>(red, plain, a...); break;
   }
@@ -44,7 +44,7 @@ template <template <int, bool, bool> class Fam, bool PLAIN>
 void configure_family(int lim) {
   switch (lim) {
     case LIM_MINMOD: configure_lim<Fam, PLAIN, LIM_MINMOD>(); break;
-    case LIM_MC1: configure_lim<Fam, PLAIN, LIM_MC1>(); break;
+    case LIM_MC: configure_lim<Fam, PLAIN, LIM_MC>(); break;
     case LIM_VANLEER: configure_lim<Fam, PLAIN, LIM_VANLEER>(); break;
     default: configure_lim<Fam, PLAIN, 0>(); break;
   }

@@ -84,11 +84,13 @@ inline int march_chunk(const Grid& g, int copies) {
   }
   return best;
 }
-// the limiter code a stage's kernel is compiled for: minmod, MC with theta = 1 (LIM_MC1),
-// van Leer; 0 when the kernel reads limiter, theta and reconstruction order from the arguments
+// the limiter code a stage's kernel is compiled for: minmod, MC, van Leer; 0 when the kernel reads
+// limiter and reconstruction order from the arguments (a switch per slope).  MC with theta = 1 is
+// minmod: the central difference is the mean of the one-sided ones, and rounding is monotonic, so
+// (qp - qm)/2 is never the smallest of the three in magnitude.
 inline int compiled_limiter(int limiter, bool constant_recon, double theta) {
   if (constant_recon) return 0;
-  if (limiter == LIM_MC) return theta == 1.0 ? LIM_MC1 : 0;
+  if (limiter == LIM_MC) return theta == 1.0 ? LIM_MINMOD : LIM_MC;
   return (limiter == LIM_MINMOD || limiter == LIM_VANLEER) ? limiter : 0;
 }
 // opt the kernels of a limiter into their dynamic shared memory (the current device; a handle or
