@@ -601,27 +601,28 @@ int timed_launch(fgpu_handle* h, int kind, double bytes, F&& fn) {
 }
 
 // Viscous source of the stage state of A into h->d_visc (sources_viscosity.f90:484-507); the
-// stage kernel reads it.  Tiles: 2D 32 x 8, 3D 8 x 8 x 4.
-template <int ND> struct ViscShape;
-template <> struct ViscShape<2> { static constexpr int TX = 32, TY = 8, TZ = 1; };
-template <> struct ViscShape<3> { static constexpr int TX = 8, TY = 8, TZ = 4; };
-template <int ND, bool EU>
-void configure_visc_t() {
-  using S = ViscShape<ND>;
-  cudaFuncSetAttribute(visc_kernel<ND, EU, S::TX, S::TY, S::TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)ViscTile<ND, S::TX, S::TY, S::TZ>::SMEM);
+// stage kernel reads it.  2D: 32 x 8 tiles; 3D: 32 x 8 tiles marching in z.
+constexpr int kViscTX = 32, kViscTY = 8;   // 2D tile
+template <bool EU>
+void configure_visc_t(int nd) {
+  if (nd == 2)
+    cudaFuncSetAttribute(visc_kernel<EU, kViscTX, kViscTY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)ViscTile<kViscTX, kViscTY>::SMEM);
+  else
+    cudaFuncSetAttribute(visc_march_kernel<EU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ViscMarch::SMEM);
 }
-void configure_visc(int nd, bool e) {
-  if (nd == 2) e ? configure_visc_t<2, true>() : configure_visc_t<2, false>();
-  else e ? configure_visc_t<3, true>() : configure_visc_t<3, false>();
-}
-template <int ND, bool EU>
+void configure_visc(int nd, bool e) { e ? configure_visc_t<true>(nd) : configure_visc_t<false>(nd); }
+template <bool EU>
 void launch_visc_t(fgpu_handle* h, const ViscArgs& V) {
-  using S = ViscShape<ND>;
   const Grid& g = h->g;
-  dim3 grid((g.nx + S::TX - 1) / S::TX, (g.ny + S::TY - 1) / S::TY, ND == 3 ? (g.nz + S::TZ - 1) / S::TZ : 1);
-  visc_kernel<ND, EU, S::TX, S::TY, S::TZ>
-      <<<grid, S::TX * S::TY * S::TZ, ViscTile<ND, S::TX, S::TY, S::TZ>::SMEM, h->stream>>>(V);
+  if (h->nd == 2) {
+    const dim3 grid((g.nx + kViscTX - 1) / kViscTX, (g.ny + kViscTY - 1) / kViscTY);
+    visc_kernel<EU, kViscTX, kViscTY><<<grid, kViscTX * kViscTY, ViscTile<kViscTX, kViscTY>::SMEM, h->stream>>>(V);
+  } else {
+    using S = ViscMarch;
+    const dim3 grid((g.nx + S::TX - 1) / S::TX, (g.ny + S::TY - 1) / S::TY, (g.nz + h->kchunk - 1) / h->kchunk);
+    visc_march_kernel<EU><<<grid, S::NT, S::SMEM, h->stream>>>(V, h->kchunk);
+  }
 }
 // UpdateViscosity of the state S at the time `when` (ALPHA/BETA/POWERLAW): the conditional
 // update of the cell viscosities, then the record of its time
@@ -702,8 +703,7 @@ int launch_visc(fgpu_handle* h, const StateRef& S, int gate = 0) {
   // algorithmic bytes: the state read once, the source written once
   const double bytes = (double)(h->V + h->nd + (h->euler ? 1 : 0)) * (double)h->g.n * 8.0;
   return timed_launch(h, 1, bytes, [&] {
-    if (h->nd == 2) h->euler ? launch_visc_t<2, true>(h, V) : launch_visc_t<2, false>(h, V);
-    else h->euler ? launch_visc_t<3, true>(h, V) : launch_visc_t<3, false>(h, V);
+    h->euler ? launch_visc_t<true>(h, V) : launch_visc_t<false>(h, V);
     CUDA_TRY(h, cudaGetLastError());
     return FGPU_OK;
   });

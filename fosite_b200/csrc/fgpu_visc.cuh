@@ -68,7 +68,12 @@ __device__ __forceinline__ void interior_rv(const StateRef& S, const Grid& g, lo
     if (g.fdir == 1) rv[1] = m;
     else rv[2] = m;
   }
+#ifdef FGPU_EXACT
   const double inv_rho = 1. / rv[0];
+#else
+  double inv_rho = rcp_refined(rv[0]);
+  if (!in_range<1000, 1000>(rv[0])) inv_rho = rcp_ieee(rv[0]);
+#endif
 #pragma unroll
   for (int m = 1; m <= ND; ++m) rv[m] = rv[m] * inv_rho;
 }
@@ -84,113 +89,91 @@ __device__ __forceinline__ double div3d(double aW, double aE, double aS, double 
          cxyx * TyxC + cxzx * TzxC - cyxy * TyyC - czxz * TzzC;
 }
 
-template <int ND, int TX, int TY, int TZ>
+// 2D tile: velocities within two steps of the tile, stresses within one
+template <int TX, int TY>
 struct ViscTile {
-  static constexpr int HZ = ND == 3 ? 2 : 0, HB = ND == 3 ? 1 : 0;
-  static constexpr int VX = TX + 4, VY = TY + 4, VZ = TZ + 2 * HZ;   // velocity box
-  static constexpr int BX = TX + 2, BY = TY + 2, BZ = TZ + 2 * HB;   // stress box
-  static constexpr int NB = ND == 3 ? 6 : 3;                          // xx yy (zz) xy (xz yz)
-  static constexpr size_t SMEM = sizeof(double) * ((size_t)ND * VX * VY * VZ + (size_t)NB * BX * BY * BZ);
+  static constexpr int VX = TX + 4, VY = TY + 4;   // velocity box
+  static constexpr int BX = TX + 2, BY = TY + 2;   // stress box (xx yy xy)
+  static constexpr size_t SMEM = sizeof(double) * ((size_t)2 * VX * VY + (size_t)3 * BX * BY);
 };
 
 // steps outside [0, e) along one axis
 __device__ __forceinline__ int outside(int a, int e) { return a < 0 ? -a : (a >= e ? a - e + 1 : 0); }
 
-template <int ND, bool EU, int TX, int TY, int TZ>
-__global__ void __launch_bounds__(TX* TY* TZ) visc_kernel(const __grid_constant__ ViscArgs A) {
-  using CE = Cells<ND, EU>;
-  using L = ViscTile<ND, TX, TY, TZ>;
-  constexpr int V = Phys<ND, EU>::V;
-  constexpr int NT = TX * TY * TZ;
-  constexpr int VX = L::VX, VY = L::VY, VZ = L::VZ, BX = L::BX, BY = L::BY, BZ = L::BZ;
-  extern __shared__ __align__(16) double visc_smem[];
-  if (A.gate && (A.ctl->stop | A.ctl->brk)) return;
-  if (gated_out(A.ctl, A.gate)) return;
-  double* const Vs = visc_smem;                     // [ND][VZ][VY][VX]
-  double* const Ts = Vs + ND * VX * VY * VZ;        // [NB][BZ][BY][BX]
-  const Grid& g = A.g;
-  const MetricP& M = A.mt;
-  const int i0 = blockIdx.x * TX, j0 = blockIdx.y * TY, k0 = ND == 3 ? blockIdx.z * TZ : 0;
-  const int ex = min(TX, g.nx - i0), ey = min(TY, g.ny - j0), ez = ND == 3 ? min(TZ, g.nz - k0) : 1;
-  auto VV = [&](int m, int a, int b, int c) -> double& {   // velocity at tile-local (a, b, c)
-    return Vs[((m * VZ + (c + L::HZ)) * VY + (b + 2)) * VX + (a + 2)];
-  };
-  auto TT = [&](int q, int a, int b, int c) -> double& {   // stress component q at tile-local (a, b, c)
-    return Ts[((q * BZ + (c + L::HB)) * BY + (b + 1)) * BX + (a + 1)];
-  };
+// The face ghost behind one periodic face is the wrapped interior cell (face_ghost_p): wraps the
+// coordinates; false when the cell is interior, or a ghost of another kind.
+__device__ __forceinline__ bool wrap_face(const Grid& g, int nd, int& i, int& j, int& k) {
+  const bool xo = i < 0 || i >= g.nx, yo = j < 0 || j >= g.ny, zo = nd == 3 && (k < 0 || k >= g.nz);
+  if (xo + yo + zo != 1) return false;
+  int& x = xo ? i : yo ? j : k;
+  const int n = xo ? g.nx : yo ? g.ny : g.nz;
+  const bool lo = x < 0;
+  if (g.bc[(xo ? 0 : yo ? 2 : 4) + (lo ? 0 : 1)] != BC_PERIODIC) return false;
+  x += lo ? n : -n;
+  return true;
+}
 
-  // ---- phase 1: primitive velocity of the ghost-padded state within two steps of the tile
-  for (int t = threadIdx.x; t < VX * VY * VZ; t += NT) {
-    const int lx = t % VX, r = t / VX, ly = r % VY, lz = r / VY;
-    const int a = lx - 2, b = ly - 2, c = lz - L::HZ;
-    const int ox = outside(a, ex), oy = outside(b, ey), oz = ND == 3 ? outside(c, ez) : 0;
-    if (ox + oy + oz > 2) continue;
-    const int gi = i0 + a, gj = j0 + b, gk = ND == 3 ? k0 + c : 0;
-    double p[V];
-    if (gi >= 0 && gi < g.nx && gj >= 0 && gj < g.ny && gk >= 0 && gk < g.nz)
-      interior_rv<ND>(A.in, g, CE::lin(g, gi, gj, gk), gi, gj, p);
-    else
-      CE::cell_p(A.in, g, A.ph, M, gi, gj, gk, p);
-#pragma unroll
-    for (int m = 0; m < ND; ++m) Vs[((m * VZ + lz) * VY + ly) * VX + lx] = p[1 + m];
+// A difference over a cell width: the quotient (exact build) or the product with the width's
+// inverse, one reciprocal per cell and direction instead of nine divisions.
+__device__ __forceinline__ double width_inverse(double d) {
+#ifdef FGPU_EXACT
+  return d;
+#else
+  return rcp_refined(d);
+#endif
+}
+__device__ __forceinline__ double over(double x, double d, double rd) {
+#ifdef FGPU_EXACT
+  return x / d;
+#else
+  return x * rd;
+#endif
+}
+
+// CalcStresses of cell (a, b, c) (sources_viscosity.f90, mesh_midpoint.f90:156-183, 474-502): VV(m, ...)
+// reads velocities, TT(q, ...) is the stress component q
+template <int ND, class FV, class FT>
+__device__ __forceinline__ void visc_stress(const MetricP& M, int ip, double eta, double mub, int a, int b, int c,
+                                            FV&& VV, FT&& TT) {
+  const double dlx = M.dlx[ip], dly = M.dly[ip], rdlx = width_inverse(dlx), rdly = width_inverse(dly);
+  const double cxyx = M.cxyx[ip], cyxy = M.cyxy[ip];
+  const double vx = VV(0, a, b, c), vy = VV(1, a, b, c);
+  const double vxW = VV(0, a - 1, b, c), vxE = VV(0, a + 1, b, c), vxS = VV(0, a, b - 1, c), vxN = VV(0, a, b + 1, c);
+  const double vyW = VV(1, a - 1, b, c), vyE = VV(1, a + 1, b, c), vyS = VV(1, a, b - 1, c), vyN = VV(1, a, b + 1, c);
+  if (ND == 2) {
+    // VectorDivergence2D_1 of v (mesh_midpoint.f90:156-183) times the bulk viscosity
+    const double tb = mub * div3d(M.dAxW[ip], M.dAxE[ip], M.dAyS[ip], M.dAyS[ip], 0.0, 0.0, M.dydzdV[ip],
+                                    M.dzdxdV[ip], 0.0, 0.0, 0.0, 0.0, 0.0, 0.5 * (vxW + vx), 0.5 * (vxE + vx),
+                                    0.5 * (vyS + vy), 0.5 * (vyN + vy), 0.0, 0.0, 0.0, 0.0, 0.0, 0.0);
+    TT(0, a, b, c) = eta * (over((vxE - vxW), dlx, rdlx) + 2.0 * cxyx * vy) + tb;
+    TT(1, a, b, c) = eta * (over((vyN - vyS), dly, rdly) + 2.0 * cyxy * vx) + tb;
+    TT(2, a, b, c) = eta * (0.5 * (over((vyE - vyW), dlx, rdlx) + over((vxN - vxS), dly, rdly)) - cxyx * vx - cyxy * vy);
+  } else {
+    const double dlz = M.dlz[ip], rdlz = width_inverse(dlz);
+    const double cxzx = M.cxzx[ip], cyzy = M.cyzy[ip], czxz = M.czxz[ip], czyz = M.czyz[ip];
+    const double vz = VV(2, a, b, c);
+    const double vxB = VV(0, a, b, c - 1), vxT = VV(0, a, b, c + 1), vyB = VV(1, a, b, c - 1), vyT = VV(1, a, b, c + 1);
+    const double vzW = VV(2, a - 1, b, c), vzE = VV(2, a + 1, b, c), vzS = VV(2, a, b - 1, c), vzN = VV(2, a, b + 1, c);
+    const double vzB = VV(2, a, b, c - 1), vzT = VV(2, a, b, c + 1);
+    // VectorDivergence3D (mesh_midpoint.f90:474-502)
+    const double tb = mub * div3d(M.dAxW[ip], M.dAxE[ip], M.dAyS[ip], M.dAyS[ip], M.dAzB[ip], M.dAzB[ip],
+                                    M.dydzdV[ip], M.dzdxdV[ip], M.dxdydV[ip], 0.0, 0.0, 0.0, 0.0,
+                                    0.5 * (vxW + vx), 0.5 * (vxE + vx), 0.5 * (vyS + vy), 0.5 * (vyN + vy),
+                                    0.5 * (vzB + vz), 0.5 * (vzT + vz), 0.0, 0.0, 0.0, 0.0);
+    TT(0, a, b, c) = eta * (over((vxE - vxW), dlx, rdlx) + 2.0 * cxyx * vy + 2.0 * cxzx * vz) + tb;
+    TT(1, a, b, c) = eta * (over((vyN - vyS), dly, rdly) + 2.0 * cyxy * vx + 2.0 * cyzy * vz) + tb;
+    TT(2, a, b, c) = eta * (over((vzT - vzB), dlz, rdlz) + 2.0 * czxz * vx + 2.0 * czyz * vy) + tb;
+    TT(3, a, b, c) = eta * (0.5 * (over((vyE - vyW), dlx, rdlx) + over((vxN - vxS), dly, rdly)) - cxyx * vx - cyxy * vy);
+    TT(4, a, b, c) = eta * (0.5 * (over((vzE - vzW), dlx, rdlx) + over((vxT - vxB), dlz, rdlz)) - czxz * vz - cxzx * vx);
+    TT(5, a, b, c) = eta * (0.5 * (over((vyT - vyB), dlz, rdlz) + over((vzN - vzS), dly, rdly)) - czyz * vz - cyzy * vy);
   }
-  __syncthreads();
-
-  // ---- phase 2: CalcStresses within one step of the tile (the interior and the first ghost layer)
-  for (int t = threadIdx.x; t < BX * BY * BZ; t += NT) {
-    const int lx = t % BX, r = t / BX, ly = r % BY, lz = r / BY;
-    const int a = lx - 1, b = ly - 1, c = lz - L::HB;
-    if (outside(a, ex) + outside(b, ey) + (ND == 3 ? outside(c, ez) : 0) > 1) continue;
-    const int ip = i0 + a + 2;
-    const double dlx = M.dlx[ip], dly = M.dly[ip];
-    const double cxyx = M.cxyx[ip], cyxy = M.cyxy[ip];
-    double eta = A.eta, mub = A.mub;
-    if (A.dynvis) {
-      eta = A.dynvis[pad_index<ND>(g, i0 + a, j0 + b, ND == 3 ? k0 + c : 0)];
-      mub = -2. / 3. * eta;
-    }
-    const double vx = VV(0, a, b, c), vy = VV(1, a, b, c);
-    const double vxW = VV(0, a - 1, b, c), vxE = VV(0, a + 1, b, c), vxS = VV(0, a, b - 1, c), vxN = VV(0, a, b + 1, c);
-    const double vyW = VV(1, a - 1, b, c), vyE = VV(1, a + 1, b, c), vyS = VV(1, a, b - 1, c), vyN = VV(1, a, b + 1, c);
-    if (ND == 2) {
-      // VectorDivergence2D_1 of v (mesh_midpoint.f90:156-183) times the bulk viscosity
-      const double tb = mub * div3d(M.dAxW[ip], M.dAxE[ip], M.dAyS[ip], M.dAyS[ip], 0.0, 0.0, M.dydzdV[ip],
-                                      M.dzdxdV[ip], 0.0, 0.0, 0.0, 0.0, 0.0, 0.5 * (vxW + vx), 0.5 * (vxE + vx),
-                                      0.5 * (vyS + vy), 0.5 * (vyN + vy), 0.0, 0.0, 0.0, 0.0, 0.0, 0.0);
-      TT(0, a, b, c) = eta * ((vxE - vxW) / dlx + 2.0 * cxyx * vy) + tb;
-      TT(1, a, b, c) = eta * ((vyN - vyS) / dly + 2.0 * cyxy * vx) + tb;
-      TT(2, a, b, c) = eta * (0.5 * ((vyE - vyW) / dlx + (vxN - vxS) / dly) - cxyx * vx - cyxy * vy);
-    } else {
-      const double dlz = M.dlz[ip];
-      const double cxzx = M.cxzx[ip], cyzy = M.cyzy[ip], czxz = M.czxz[ip], czyz = M.czyz[ip];
-      const double vz = VV(2, a, b, c);
-      const double vxB = VV(0, a, b, c - 1), vxT = VV(0, a, b, c + 1), vyB = VV(1, a, b, c - 1), vyT = VV(1, a, b, c + 1);
-      const double vzW = VV(2, a - 1, b, c), vzE = VV(2, a + 1, b, c), vzS = VV(2, a, b - 1, c), vzN = VV(2, a, b + 1, c);
-      const double vzB = VV(2, a, b, c - 1), vzT = VV(2, a, b, c + 1);
-      // VectorDivergence3D (mesh_midpoint.f90:474-502)
-      const double tb = mub * div3d(M.dAxW[ip], M.dAxE[ip], M.dAyS[ip], M.dAyS[ip], M.dAzB[ip], M.dAzB[ip],
-                                      M.dydzdV[ip], M.dzdxdV[ip], M.dxdydV[ip], 0.0, 0.0, 0.0, 0.0,
-                                      0.5 * (vxW + vx), 0.5 * (vxE + vx), 0.5 * (vyS + vy), 0.5 * (vyN + vy),
-                                      0.5 * (vzB + vz), 0.5 * (vzT + vz), 0.0, 0.0, 0.0, 0.0);
-      TT(0, a, b, c) = eta * ((vxE - vxW) / dlx + 2.0 * cxyx * vy + 2.0 * cxzx * vz) + tb;
-      TT(1, a, b, c) = eta * ((vyN - vyS) / dly + 2.0 * cyxy * vx + 2.0 * cyzy * vz) + tb;
-      TT(2, a, b, c) = eta * ((vzT - vzB) / dlz + 2.0 * czxz * vx + 2.0 * czyz * vy) + tb;
-      TT(3, a, b, c) = eta * (0.5 * ((vyE - vyW) / dlx + (vxN - vxS) / dly) - cxyx * vx - cyxy * vy);
-      TT(4, a, b, c) = eta * (0.5 * ((vzE - vzW) / dlx + (vxT - vxB) / dlz) - czxz * vz - cxzx * vx);
-      TT(5, a, b, c) = eta * (0.5 * ((vyT - vyB) / dlz + (vzN - vzS) / dly) - czyz * vz - cyzy * vy);
-    }
-  }
-  __syncthreads();
-
-  // ---- phase 3: tensor divergence (and the heating) of the own cell
-  const int a = threadIdx.x % TX, b = (threadIdx.x / TX) % TY, c = ND == 3 ? threadIdx.x / (TX * TY) : 0;
-  if (a >= ex || b >= ey || c >= ez) return;
-  const int ip = i0 + a + 2;
-  const long long idx = CE::lin(g, i0 + a, j0 + b, k0 + c);
+}
+// The tensor divergence (and the heating) of cell (a, b, c) into sv
+template <int ND, bool EU, class FV, class FT>
+__device__ __forceinline__ void visc_source(const MetricP& M, int ip, int a, int b, int c, FV&& VV, FT&& TT, double* sv) {
   const double aW = M.dAxW[ip], aE = M.dAxE[ip], aS = M.dAyS[ip];
   const double dydzdV = M.dydzdV[ip], dzdxdV = M.dzdxdV[ip];
   const double cxyx = M.cxyx[ip], cyxy = M.cyxy[ip];
-  double sv[ND + 1];
   if (ND == 2) {
     const double xx = TT(0, a, b, c), yy = TT(1, a, b, c), xy = TT(2, a, b, c);
     // TensorDivergence2D_1 (mesh_midpoint.f90:283-323) with Tyx = Txy
@@ -245,8 +228,144 @@ __global__ void __launch_bounds__(TX* TY* TZ) visc_kernel(const __grid_constant_
                     0.5 * (row(4, 5, 2, 0, 0, -1) + tz), 0.5 * (row(4, 5, 2, 0, 0, 1) + tz), 0.0, 0.0, 0.0, 0.0);
     }
   }
+}
+
+template <bool EU, int TX, int TY>
+__global__ void __launch_bounds__(TX* TY) visc_kernel(const __grid_constant__ ViscArgs A) {
+  using CE = Cells<2, EU>;
+  using L = ViscTile<TX, TY>;
+  constexpr int V = Phys<2, EU>::V;
+  constexpr int NT = TX * TY;
+  constexpr int VX = L::VX, VY = L::VY, BX = L::BX, BY = L::BY;
+  extern __shared__ __align__(16) double visc_smem[];
+  if (A.gate && (A.ctl->stop | A.ctl->brk)) return;
+  if (gated_out(A.ctl, A.gate)) return;
+  double* const Vs = visc_smem;                // [2][VY][VX]
+  double* const Ts = Vs + 2 * VX * VY;         // [3][BY][BX]
+  const Grid& g = A.g;
+  const MetricP& M = A.mt;
+  const int i0 = blockIdx.x * TX, j0 = blockIdx.y * TY;
+  const int ex = min(TX, g.nx - i0), ey = min(TY, g.ny - j0);
+  auto VV = [&](int m, int a, int b, int) -> double& { return Vs[(m * VY + (b + 2)) * VX + (a + 2)]; };
+  auto TT = [&](int q, int a, int b, int) -> double& { return Ts[(q * BY + (b + 1)) * BX + (a + 1)]; };
+
+  // ---- primitive velocity of the ghost-padded state within two steps of the tile
+  for (int t = threadIdx.x; t < VX * VY; t += NT) {
+    const int a = t % VX - 2, b = t / VX - 2;
+    if (outside(a, ex) + outside(b, ey) > 2) continue;
+    int gi = i0 + a, gj = j0 + b, gk = 0;
+    double p[V];
+    // (with frame changes the wrapped cell's own apply: fargo_ix of its coordinates)
+    if ((gi >= 0 && gi < g.nx && gj >= 0 && gj < g.ny) || wrap_face(g, 2, gi, gj, gk))
+      interior_rv<2>(A.in, g, CE::lin(g, gi, gj, 0), gi, gj, p);
+    else
+      CE::cell_p(A.in, g, A.ph, M, gi, gj, 0, p);
+    VV(0, a, b, 0) = p[1];
+    VV(1, a, b, 0) = p[2];
+  }
+  __syncthreads();
+
+  // ---- CalcStresses within one step of the tile (the interior and the first ghost layer)
+  for (int t = threadIdx.x; t < BX * BY; t += NT) {
+    const int a = t % BX - 1, b = t / BX - 1;
+    if (outside(a, ex) + outside(b, ey) > 1) continue;
+    double eta = A.eta, mub = A.mub;
+    if (A.dynvis) {
+      eta = A.dynvis[pad_index<2>(g, i0 + a, j0 + b, 0)];
+      mub = -2. / 3. * eta;
+    }
+    visc_stress<2>(M, i0 + a + 2, eta, mub, a, b, 0, VV, TT);
+  }
+  __syncthreads();
+
+  // ---- tensor divergence (and the heating) of the own cell
+  const int a = threadIdx.x % TX, b = threadIdx.x / TX;
+  if (a >= ex || b >= ey) return;
+  const long long idx = CE::lin(g, i0 + a, j0 + b, 0);
+  double sv[3];
+  visc_source<2, EU>(M, i0 + a + 2, a, b, 0, VV, TT, sv);
 #pragma unroll
-  for (int m = 0; m < ND + (EU ? 1 : 0); ++m) A.out[(long long)m * g.n + idx] = sv[m];
+  for (int m = 0; m < 2 + (EU ? 1 : 0); ++m) A.out[(long long)m * g.n + idx] = sv[m];
+}
+
+// 3D meshes: a 32 x 8 tile marches a chunk of z.  Each plane's velocities (tile and two halo cells,
+// without the far corners) and stresses (one halo cell) are formed once and kept in rings of five and
+// three planes, so that a cell costs 1.7 velocity conversions and 1.3 stress tensors.  (An 8 x 8 x 4
+// tile forms 4.5 and 2.3 of them: 135 us at 96^3 against 112 us.)  Bound by the latency of its chains
+// between two barriers a plane: 33% issue activity at 16 warps an SM.
+struct ViscMarch {
+  static constexpr int TX = 32, TY = 8, NT = TX * TY;
+  static constexpr int VX = TX + 4, VY = TY + 4, NV = 5;
+  static constexpr int BX = TX + 2, BY = TY + 2, NS = 3;
+  static constexpr size_t SMEM = sizeof(double) * ((size_t)NV * 3 * VX * VY + (size_t)NS * 6 * BX * BY);
+};
+template <bool EU>
+__global__ void __launch_bounds__(ViscMarch::NT, 2) visc_march_kernel(const __grid_constant__ ViscArgs A, const int kchunk) {
+  using CE = Cells<3, EU>;
+  using L = ViscMarch;
+  constexpr int V = Phys<3, EU>::V;
+  extern __shared__ __align__(16) double visc_smem[];
+  if (A.gate && (A.ctl->stop | A.ctl->brk)) return;
+  if (gated_out(A.ctl, A.gate)) return;
+  double* const Vs = visc_smem;                              // [NV][3][VY][VX]
+  double* const Ts = Vs + L::NV * 3 * L::VX * L::VY;         // [NS][6][BY][BX]
+  const Grid& g = A.g;
+  const MetricP& M = A.mt;
+  const int i0 = blockIdx.x * L::TX, j0 = blockIdx.y * L::TY, k0 = blockIdx.z * kchunk;
+  const int ex = min(L::TX, g.nx - i0), ey = min(L::TY, g.ny - j0), k1 = min(g.nz, k0 + kchunk);
+  auto VV = [&](int m, int a, int b, int c) -> double& {   // velocity at tile-local (a, b), plane c
+    return Vs[((((c - k0 + 2) % L::NV) * 3 + m) * L::VY + b + 2) * L::VX + a + 2];
+  };
+  auto TT = [&](int q, int a, int b, int c) -> double& {   // stress component q at (a, b), plane c
+    return Ts[((((c - k0 + 1) % L::NS) * 6 + q) * L::BY + b + 1) * L::BX + a + 1];
+  };
+  // the cells of plane c that a stress or source reads lie within two steps of the tile in all
+  auto velocities = [&](int c) {
+    const int oz = outside(c - k0, k1 - k0);
+    for (int t = threadIdx.x; t < L::VX * L::VY; t += L::NT) {
+      const int a = t % L::VX - 2, b = t / L::VX - 2;
+      if (outside(a, ex) + outside(b, ey) + oz > 2) continue;
+      int gi = i0 + a, gj = j0 + b, gk = c;
+      double p[V];
+      if ((gi >= 0 && gi < g.nx && gj >= 0 && gj < g.ny && gk >= 0 && gk < g.nz) || wrap_face(g, 3, gi, gj, gk))
+        interior_rv<3>(A.in, g, CE::lin(g, gi, gj, gk), gi, gj, p);
+      else
+        CE::cell_p(A.in, g, A.ph, M, gi, gj, gk, p);
+#pragma unroll
+      for (int m = 0; m < 3; ++m) VV(m, a, b, c) = p[1 + m];
+    }
+  };
+  auto stresses = [&](int c) {
+    const int oz = outside(c - k0, k1 - k0);
+    for (int t = threadIdx.x; t < L::BX * L::BY; t += L::NT) {
+      const int a = t % L::BX - 1, b = t / L::BX - 1;
+      if (outside(a, ex) + outside(b, ey) + oz > 1) continue;
+      double eta = A.eta, mub = A.mub;
+      if (A.dynvis) {
+        eta = A.dynvis[pad_index<3>(g, i0 + a, j0 + b, c)];
+        mub = -2. / 3. * eta;
+      }
+      visc_stress<3>(M, i0 + a + 2, eta, mub, a, b, c, VV, TT);
+    }
+  };
+  // passes k0 - 4 .. k0 - 1 fill the rings
+  const int a = threadIdx.x % L::TX, b = threadIdx.x / L::TX;
+#pragma unroll 1
+  for (int k = k0 - 4; k < k1; ++k) {
+    velocities(k + 2);   // its slot held plane k - 3, which no pass since the last barrier reads
+    if (k < k0 - 2) continue;
+    __syncthreads();
+    stresses(k + 1);
+    if (k < k0) continue;
+    __syncthreads();
+    if (a < ex && b < ey) {
+      double sv[4];
+      visc_source<3, EU>(M, i0 + a + 2, a, b, k, VV, TT, sv);
+      const long long idx = CE::lin(g, i0 + a, j0 + b, k);
+#pragma unroll
+      for (int m = 0; m < 3 + (EU ? 1 : 0); ++m) A.out[(long long)m * g.n + idx] = sv[m];
+    }
+  }
 }
 
 // ---------------------------------------------------------------- ALPHA / BETA / POWERLAW
