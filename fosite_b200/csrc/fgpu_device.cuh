@@ -594,7 +594,11 @@ struct Cells {
       double v = p[1 + m];
       double mn = dmin(0., v - cs), mx = dmax(0., v + cs);
       w[m] = dmax(mx, -mn);
+#ifdef FGPU_EXACT
       a[m] = w[m] / dl[m];
+#else
+      a[m] = w[m] * rcp_refined(dl[m]);
+#endif
     }
     if (ND == 2) { out[0] = a[0] + a[1]; out[1] = 0.0; out[2] = 0.0; }
     else { out[0] = a[0]; out[1] = a[1]; out[2] = a[2]; }

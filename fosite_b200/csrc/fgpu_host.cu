@@ -1699,6 +1699,13 @@ int fgpu_create(const fgpu_config* cfg, int device, fgpu_handle** out) {
   }
   if (!rc) {
     // FGPU_STAGE_VARIANT / FGPU_KCHUNK force a stage-kernel layout and z chunk (the tuner's choice otherwise)
+    // Default layout: the marching kernels (0).  2D isothermal grids start with the register-capped
+    // shared-memory tile (3): their rows carry a third less arithmetic while the opening of a warp's
+    // chunk costs the same, so that small disks are faster on tiles (186 x 390: 44 against 52 us a
+    // step), 512 x 1024 with FARGO is a draw (195 us), and only large ones gain from marching (48
+    // disks in one batch, 5 million cells: 950 against 1430 us), which the tuner finds.  One layout for
+    // all of them, so that a batch and its members' lone runs keep the same bits.
+    h->variant = (!h->euler && h->nd == 2) ? 3 : 0;
     if (const char* e = std::getenv("FGPU_STAGE_VARIANT")) h->variant = std::max(0, std::min(7, std::atoi(e)));
     if (const char* e = std::getenv("FGPU_KCHUNK")) { int v = std::atoi(e); if (v > 0) h->kchunk = v; }
     if (const char* e = std::getenv("FGPU_MATERIALIZE")) h->materialize = std::atoi(e) != 0;

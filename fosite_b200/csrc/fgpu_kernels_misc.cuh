@@ -37,29 +37,36 @@ __device__ __forceinline__ void to_comoving(const double* w_sub, const Grid& g, 
   }
 }
 
-// ghost cell number t -> padded coordinates (x slabs, then y slabs, then z slabs)
+// ghost cell number t -> padded coordinates (x slabs, then y slabs, then z slabs); 32-bit
+// arithmetic: the surface of a grid that fits the device has fewer than 2^31 ghost cells
 template <int ND>
-__device__ __forceinline__ void ghost_coords(const Grid& g, long long t, int& px, int& py, int& pz) {
-  const int NXp = g.nx + 4, NYp = g.ny + 4, NZp = ND == 3 ? g.nz + 4 : 1;
-  long long nxs = 4LL * NYp * NZp;
+__device__ __forceinline__ void ghost_coords(const Grid& g, long long t64, int& px, int& py, int& pz) {
+  const unsigned NXp = g.nx + 4, NYp = g.ny + 4, NZp = ND == 3 ? g.nz + 4 : 1;
+  unsigned t = (unsigned)t64;
+  const unsigned nxs = 4u * NYp * NZp;
   if (t < nxs) {
-    int q = (int)(t % 4); long long r = t / 4;
-    px = q < 2 ? q : NXp - 4 + q;
-    py = (int)(r % NYp); pz = (int)(r / NYp);
+    const int q = (int)(t % 4);
+    const unsigned r = t / 4;
+    px = q < 2 ? q : (int)NXp - 4 + q;
+    if (ND == 3) { py = (int)(r % NYp); pz = (int)(r / NYp); }
+    else { py = (int)r; pz = 0; }
     return;
   }
   t -= nxs;
-  long long nys = 4LL * g.nx * NZp;
-  if (t < nys) {
-    int q = (int)(t % 4); long long r = t / 4;
-    py = q < 2 ? q : NYp - 4 + q;
-    px = 2 + (int)(r % g.nx); pz = (int)(r / g.nx);
+  const unsigned nys = 4u * g.nx * NZp;
+  if (ND == 2 || t < nys) {
+    const int q = (int)(t % 4);
+    const unsigned r = t / 4;
+    py = q < 2 ? q : (int)NYp - 4 + q;
+    if (ND == 3) { px = 2 + (int)(r % (unsigned)g.nx); pz = (int)(r / (unsigned)g.nx); }
+    else { px = 2 + (int)r; pz = 0; }
     return;
   }
   t -= nys;
-  int q = (int)(t % 4); long long r = t / 4;
-  pz = q < 2 ? q : NZp - 4 + q;
-  px = 2 + (int)(r % g.nx); py = 2 + (int)(r / g.nx);
+  const int q = (int)(t % 4);
+  const unsigned r = t / 4;
+  pz = q < 2 ? q : (int)NZp - 4 + q;
+  px = 2 + (int)(r % (unsigned)g.nx); py = 2 + (int)(r / (unsigned)g.nx);
 }
 
 // The step's closing scalar work, run by the last block of the boundary pass:
