@@ -1,0 +1,72 @@
+"""State transfers: the pinned lanes of large pageable arrays, the driver's path of small and pinned
+ones, and transfers of several threads at once give back what was uploaded, byte for byte."""
+import threading
+
+import numpy as np
+import pytest
+
+from fosite_b200 import abi
+from cases import _gauss3d, _khi
+
+
+def _sim(case):
+    from fosite_b200.sim import Simulation
+    cfg, p, _ = case
+    s = Simulation(cfg)
+    c = np.random.default_rng(cfg.inum).uniform(1.0, 2.0, (s.vnum,) + s.shape)
+    c[-1] += 10.0
+    return s, c
+
+
+def _interior(a, cfg):
+    return a[:, 2:-2, 2:-2, 2:-2] if cfg.knum > 1 else a[:, :, 2:-2, 2:-2]
+
+
+# ghost-padded bytes: around 1 MiB (downloads take the lanes from there), 4.2 MB in odd rows, 48 and 110 MB
+# (uploads too, from 8 MiB)
+@pytest.mark.gpu
+@pytest.mark.parametrize("case", [_khi(n=(36, 36)), _khi(n=(1021, 27)), _khi(n=(252, 125)), _khi(n=(509, 251)),
+                                  _gauss3d(n=(100, 100, 106)), _gauss3d(n=(131, 133, 137))],
+                         ids=["50K", "1M-", "1M+", "4M", "48M", "110M"])
+def test_round_trip(case):
+    s, c = _sim(case)
+    for _ in range(2):
+        s.set_state(abi.CVAR, c)
+        assert np.array_equal(_interior(s.get(abi.CVAR), s.cfg), _interior(c, s.cfg))
+        c = c * 1.5
+    s.close()
+
+
+@pytest.mark.gpu
+def test_pinned_host_arrays():
+    import ctypes as C
+
+    import torch
+    s, c = _sim(_khi(n=(509, 251)))
+    src = torch.from_numpy(c).pin_memory()
+    dst = torch.empty_like(src).pin_memory()
+    s._check(s.L.fgpu_upload_state(s.h, abi.CVAR, C.c_void_p(src.data_ptr()), src.numel()))
+    s._check(s.L.fgpu_download(s.h, abi.CVAR, C.c_void_p(dst.data_ptr()), dst.numel()))
+    assert np.array_equal(_interior(dst.numpy(), s.cfg), _interior(c, s.cfg))
+    s.close()
+
+
+@pytest.mark.gpu
+def test_threads_transfer_at_once():
+    sims = [_sim(_khi(n=(509 + 2 * k, 251))) for k in range(4)]
+    bad = []
+
+    def work(s, c):
+        for _ in range(8):
+            s.set_state(abi.CVAR, c)
+            if not np.array_equal(_interior(s.get(abi.CVAR), s.cfg), _interior(c, s.cfg)):
+                bad.append(s.shape)
+
+    threads = [threading.Thread(target=work, args=sc) for sc in sims]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
+    for s, _ in sims:
+        s.close()
