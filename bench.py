@@ -542,7 +542,7 @@ def run_ensemble(args, world=1, rank=0, local=0, emit=True, steps=None):
                        "parallelism": "members dealt round-robin over %d GPU(s)" % world},
             "member_steps_per_s": members_all * args.steps / t_batch,
             "plain_loop": {"value": cells * args.steps / t_plain, "ms_per_step": 1e3 * t_plain / args.steps,
-                           "layouts": "the library's default (shared-memory tile 0)"},
+                           "layouts": "the library's default"},
             "plain_loop_tuned": {"value": cells * args.steps / t_tuned, "ms_per_step": 1e3 * t_tuned / args.steps,
                                  "layouts_rank0": {str(k): v for k, v in sorted(tuned_layouts.items())}},
             "speedup_vs_plain": t_plain / t_batch, "speedup_vs_plain_tuned": t_tuned / t_batch,

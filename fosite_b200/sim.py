@@ -287,7 +287,7 @@ class Batch:
         return int(v.value)
 
     def layout(self):
-        """The batch's stage layout (0/2/3 shared-memory tiles, 6 TMA-staged tiles)."""
+        """The batch's stage layout (0/6 the marching kernels, 2/3 shared-memory tiles)."""
         v = C.c_int(0)
         self._check(self.L.fgpu_batch_layout(self.b, C.byref(v)))
         return int(v.value)

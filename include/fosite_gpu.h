@@ -282,7 +282,8 @@ int fgpu_set_output_time(fgpu_handle* h, double tout);
  * counterpart in the reference. */
 int fgpu_autotune(fgpu_handle* h, int reps, int* variant);
 /* The stage-kernel layout later steps use (the tuner's choice, FGPU_STAGE_VARIANT, or
- * the default 0) and, for 3D grids, the z extent one block marches through.  Either
+ * the default 0: the marching kernels wherever they serve the stage, else the shared-memory
+ * base tile) and, for 3D grids, the z extent one block marches through.  Either
  * pointer may be NULL.  No counterpart in the reference. */
 int fgpu_stage_layout(const fgpu_handle* h, int* variant, int* kchunk);
 
@@ -320,10 +321,8 @@ int  fgpu_batch_run(fgpu_batch* b, int64_t nsteps, int* active);
  * updates the members' status. */
 int  fgpu_batch_enqueue(fgpu_batch* b, int64_t nsteps);
 int  fgpu_batch_collect(fgpu_batch* b, int* active);
-/* fgpu_autotune for the batched stage kernel: times the shared-memory tile layouts
- * 0, 2, 3 and, for fixed-step 2D batches whose every stage it serves, the
- * TMA-staged layout 6 (the layout the batch starts with when its first member's
- * layout is 6 or 7), and keeps the fastest. */
+/* fgpu_autotune for the batched stage kernel: times the marching kernels (layout 0) and the
+ * shared-memory tile layouts 2 and 3, and keeps the fastest. */
 int  fgpu_batch_autotune(fgpu_batch* b, int reps, int* variant);
 /* the batch's current stage layout */
 int  fgpu_batch_layout(const fgpu_batch* b, int* variant);
