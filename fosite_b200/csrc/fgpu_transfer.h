@@ -57,9 +57,12 @@ class Transfer {
     const size_t pieces = (bytes + piece - 1) / piece;
     const int n = (int)std::min<size_t>(lanes_.size(), pieces);
     std::vector<cudaError_t> err(n, cudaSuccess);
+    const cudaStreamCaptureMode capture = capture_mode();
     auto work = [&](int t) {
       Lane& L = lanes_[t];
-      cudaError_t r = cudaSetDevice(device);
+      cudaStreamCaptureMode mode = capture;   // the lane's threads wait under the caller's rules
+      cudaError_t r = cudaThreadExchangeStreamCaptureMode(&mode);
+      if (r == cudaSuccess) r = cudaSetDevice(device);
       if (r == cudaSuccess) r = cudaStreamWaitEvent(L.stream, ready_, 0);
       for (size_t p = t; p < pieces && r == cudaSuccess; p += n) {
         const size_t o = p * piece, m = std::min(piece, bytes - o);
@@ -110,6 +113,16 @@ class Transfer {
       return false;
     }
     return a.type != cudaMemoryTypeUnregistered;
+  }
+  // What the calling thread may do while another thread captures a stream: a program that captures
+  // graphs of its own (in the global mode, whose captures a wait on any stream breaks) transfers from a
+  // thread that has switched itself to the relaxed mode.
+  static cudaStreamCaptureMode capture_mode() {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) return cudaStreamCaptureModeGlobal;
+    const cudaStreamCaptureMode callers = mode;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    return callers;
   }
   // lanes on this device (the last device's are given back first)
   bool prepare(int device) {

@@ -70,3 +70,43 @@ def test_threads_transfer_at_once():
     assert not bad
     for s, _ in sims:
         s.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [(36, 36), (509, 251), (1021, 517)], ids=["50K", "4M", "17M"])
+def test_transfer_while_another_thread_captures(n):
+    """A thread in the relaxed capture mode transfers while another one captures a graph in the global
+    mode: the transfer works and the capture survives (the lanes' threads wait under the same mode)."""
+    import ctypes as C
+
+    import torch
+    torch.cuda.init()
+    L = C.CDLL([x.split()[-1] for x in open("/proc/self/maps") if "libcudart.so" in x][0])
+    relaxed, glob = C.c_int(2), 0   # cudaStreamCaptureModeRelaxed, cudaStreamCaptureModeGlobal
+    s, c = _sim(_khi(n=n))
+    stream = torch.cuda.Stream()
+    begun, finish, got = threading.Event(), threading.Event(), []
+
+    def capture():
+        graph = C.c_void_p()
+        got.append(L.cudaStreamBeginCapture(C.c_void_p(stream.cuda_stream), glob))
+        begun.set()
+        finish.wait(60)
+        got.append(L.cudaStreamEndCapture(C.c_void_p(stream.cuda_stream), C.byref(graph)))
+        if graph:
+            L.cudaGraphDestroy(graph)
+
+    other = threading.Thread(target=capture)
+    assert L.cudaThreadExchangeStreamCaptureMode(C.byref(relaxed)) == 0
+    try:
+        other.start()
+        begun.wait(60)
+        s.set_state(abi.CVAR, c)
+        back = s.get(abi.CVAR)
+    finally:
+        finish.set()
+        other.join()
+        L.cudaThreadExchangeStreamCaptureMode(C.byref(relaxed))
+    assert got == [0, 0]
+    assert np.array_equal(_interior(back, s.cfg), _interior(c, s.cfg))
+    s.close()
