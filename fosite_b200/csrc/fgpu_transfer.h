@@ -4,12 +4,17 @@
 // core: 4.8 GB/s into fresh pages (703 MB of a 256^3 state: 150 ms, thirteen of its steps).  Here up
 // to kLanes host threads, each with its own pinned slot and stream, move interleaved pieces: one
 // piece is on the bus while others are copied between pinned and pageable memory (whose page faults
-// are what a core spends its time on).  The lanes (4 MiB of pinned memory each) are shared by all
-// handles of the process: made at the first large transfer, used by one transfer at a time, freed
-// with the last handle.  Transfers below kSmallDown / kSmallUp, pinned host memory, and calls that
-// find the lanes in use or cannot make them take the driver's path.  Thresholds (16 host cores, driver
-// / lanes): downloads 1.1 MB 0.27 / 0.13 ms, 8.5 MB 1.2 / 0.43, 67 MB 14.3 / 3.6; uploads, whose pages
-// exist already, 4.3 MB 0.31 / 0.37 ms, 8.5 MB 0.61 / 0.60, 34 MB 2.9 / 1.2.
+// are what a core spends its time on).  The lanes are shared by all handles of the process, used by
+// one transfer at a time, and made at the first large transfer: pinning their slots is what they
+// cost (2 MiB in all 2 ms, 32 MiB 18 ms; freeing them 4 ms), so a slot holds the pieces asked
+// of it so far (256 KiB for transfers up to 4 MiB, 4 MiB from 64 MiB), and the lanes outlive the
+// handles: a program that opens, reads and closes one grid after another keeps them (freed with every
+// last handle they cost 35 ms a 256^2 grid).  They are given back when the last handle goes and no
+// transfer has used them since the previous time that it went; at most 32 MiB and eight streams stay.
+// Transfers below kSmallDown / kSmallUp, pinned host memory, and calls that find the lanes in use or
+// cannot make them take the driver's path.  Thresholds (16 host cores, driver / lanes): downloads
+// into fresh pages 0.5 MB 0.25 / 0.22 ms, 1.1 MB 0.54 / 0.21, 8.3 MB 4.0 / 1.0, 110 MB 52 / 9.5; uploads, whose
+// pages exist already, 4.2 MB 0.24 / 0.29 ms, 8.3 MB 0.46 / 0.43, 34 MB 3.0 / 1.2.
 #pragma once
 #include <cuda_runtime.h>
 #include <algorithm>
@@ -30,14 +35,16 @@ class Transfer {
     static Transfer* t = new Transfer;   // (never destroyed: no CUDA calls at process exit)
     return *t;
   }
-  // handles alive; the lanes go with the last
+  // handles alive
   void attach() {
     std::lock_guard<std::mutex> lock(mutex_);
     ++handles_;
   }
   void detach() {
     std::lock_guard<std::mutex> lock(mutex_);
-    if (--handles_ == 0) release();
+    if (--handles_ != 0) return;
+    if (!used_) release();
+    used_ = false;
   }
   // bytes between device memory (ready in stream order of s) and host memory; returns when the copy
   // is complete.  to_host: device to host, else host to device (later work of s sees it).
@@ -46,14 +53,14 @@ class Transfer {
     std::unique_lock<std::mutex> lock(mutex_, std::defer_lock);
     if (bytes >= (to_host ? kSmallDown : kSmallUp) && !pinned(host)) (void)lock.try_lock();
     const OnDevice on(lock.owns_lock() ? device : -1);
-    if (!lock.owns_lock() || !prepare(device)) {
+    if (!lock.owns_lock() || !prepare(device, bytes)) {
       cudaError_t e = cudaMemcpyAsync(to_host ? host : dev, to_host ? dev : host, bytes, kind, s);
       return e != cudaSuccess ? e : cudaStreamSynchronize(s);
     }
+    used_ = true;
     cudaError_t e = cudaEventRecord(ready_, s);   // the lanes start after the work enqueued on s
     if (e != cudaSuccess) return e;
-    // two pieces a lane or more
-    const size_t piece = std::min(kPiece, std::max(kLeast, (bytes / (2 * lanes_.size()) + 4095) / 4096 * 4096));
+    const size_t piece = std::min(slot_bytes_, piece_bytes(bytes, lanes_.size()));
     const size_t pieces = (bytes + piece - 1) / piece;
     const int n = (int)std::min<size_t>(lanes_.size(), pieces);
     std::vector<cudaError_t> err(n, cudaSuccess);
@@ -91,6 +98,10 @@ class Transfer {
 
  private:
   struct Lane { char* slot; cudaStream_t stream; };
+  // two pieces a lane or more
+  static size_t piece_bytes(size_t bytes, size_t lanes) {
+    return std::min(kPiece, std::max(kLeast, (bytes / (2 * lanes) + 4095) / 4096 * 4096));
+  }
   struct OnDevice {   // the calling thread's device for the length of a transfer
     int before = -1;
     explicit OnDevice(int device) {
@@ -103,8 +114,11 @@ class Transfer {
   std::mutex mutex_;
   std::vector<Lane> lanes_;
   cudaEvent_t ready_ = nullptr;
+  char* slots_ = nullptr;      // one pinned block, kLanes slots of slot_bytes_
+  size_t slot_bytes_ = 0;
   int device_ = -1;
   long long handles_ = 0;
+  bool used_ = false;          // since the last handle last went
 
   static bool pinned(const void* p) {
     cudaPointerAttributes a;
@@ -124,36 +138,41 @@ class Transfer {
     cudaThreadExchangeStreamCaptureMode(&mode);
     return callers;
   }
-  // lanes on this device (the last device's are given back first)
-  bool prepare(int device) {
-    if (device_ == device && !lanes_.empty()) return true;
-    release();
-    if (cudaEventCreateWithFlags(&ready_, cudaEventDisableTiming) != cudaSuccess) {
-      ready_ = nullptr;
-      cudaGetLastError();
-      return false;
-    }
-    device_ = device;
-    const int want = std::max(1, std::min<int>(kLanes, (int)std::thread::hardware_concurrency() / 2));
-    for (int t = 0; t < want; ++t) {
-      Lane L;
-      if (cudaMallocHost(reinterpret_cast<void**>(&L.slot), kPiece) != cudaSuccess) break;
-      if (cudaStreamCreateWithFlags(&L.stream, cudaStreamNonBlocking) != cudaSuccess) {
-        cudaFreeHost(L.slot);
-        break;
+  // lanes on this device (the last device's are given back first) with slots for pieces of a transfer
+  // of `bytes`, or smaller slots where no larger ones are to be had
+  bool prepare(int device, size_t bytes) {
+    if (device_ != device || lanes_.empty()) {
+      release();
+      if (cudaEventCreateWithFlags(&ready_, cudaEventDisableTiming) != cudaSuccess) ready_ = nullptr;
+      device_ = device;
+      const int want = std::max(1, std::min<int>(kLanes, (int)std::thread::hardware_concurrency() / 2));
+      for (int t = 0; t < want && ready_; ++t) {
+        Lane L = {nullptr, nullptr};
+        if (cudaStreamCreateWithFlags(&L.stream, cudaStreamNonBlocking) != cudaSuccess) break;
+        lanes_.push_back(L);
       }
-      lanes_.push_back(L);
     }
+    if (!lanes_.empty()) reserve(piece_bytes(bytes, lanes_.size()));
     cudaGetLastError();
-    if (lanes_.empty()) release();
-    return !lanes_.empty();
+    if (lanes_.empty() || !slots_) release();
+    return slots_ != nullptr;
+  }
+  void reserve(size_t piece) {
+    size_t want = kLeast;
+    while (want < piece) want *= 2;
+    char* block = nullptr;
+    if (want <= slot_bytes_ || cudaMallocHost(reinterpret_cast<void**>(&block), want * lanes_.size()) != cudaSuccess) return;
+    if (slots_) cudaFreeHost(slots_);
+    slots_ = block;
+    slot_bytes_ = want;
+    for (size_t t = 0; t < lanes_.size(); ++t) lanes_[t].slot = slots_ + t * want;
   }
   void release() {
-    for (Lane& L : lanes_) {
-      cudaStreamDestroy(L.stream);
-      cudaFreeHost(L.slot);
-    }
+    for (Lane& L : lanes_) cudaStreamDestroy(L.stream);
     lanes_.clear();
+    if (slots_) cudaFreeHost(slots_);
+    slots_ = nullptr;
+    slot_bytes_ = 0;
     if (ready_) cudaEventDestroy(ready_);
     ready_ = nullptr;
     device_ = -1;

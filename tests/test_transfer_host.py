@@ -1,0 +1,186 @@
+"""The pinned lanes of large transfers (fosite_b200/csrc/fgpu_transfer.h) on the host: the header compiled
+against a stand-in for the CUDA runtime that copies with memcpy and counts what it is asked for."""
+import ctypes as C
+import os
+import shutil
+import subprocess
+import tempfile
+
+import numpy as np
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CSRC = os.path.join(os.path.dirname(HERE), "fosite_b200", "csrc")
+
+RUNTIME = r'''
+#pragma once
+#include <atomic>
+#include <cstdlib>
+#include <cstring>
+typedef int cudaError_t;
+typedef struct Stream { int device; } *cudaStream_t;
+typedef struct Event { int device; } *cudaEvent_t;
+enum { cudaSuccess = 0, cudaErrorMemoryAllocation = 2 };
+enum { cudaStreamNonBlocking = 1, cudaEventDisableTiming = 2, cudaMemoryTypeUnregistered = 0 };
+enum cudaMemcpyKind { cudaMemcpyHostToDevice = 1, cudaMemcpyDeviceToHost = 2 };
+enum cudaStreamCaptureMode { cudaStreamCaptureModeGlobal, cudaStreamCaptureModeThreadLocal, cudaStreamCaptureModeRelaxed };
+struct cudaPointerAttributes { int type; };
+namespace fake {
+inline std::atomic<long long> pins{0}, frees{0}, bytes{0}, streams{0}, destroyed{0}, copies{0}, waits{0};
+inline std::atomic<long long> piece{0};   // of the largest copy
+inline thread_local int device = 0;
+inline thread_local cudaStreamCaptureMode mode = cudaStreamCaptureModeGlobal;
+struct Head { size_t n; char pad[56]; };
+}  // namespace fake
+inline cudaError_t cudaGetLastError() { return 0; }
+inline cudaError_t cudaSetDevice(int d) { fake::device = d; return 0; }
+inline cudaError_t cudaGetDevice(int* d) { *d = fake::device; return 0; }
+inline cudaError_t cudaThreadExchangeStreamCaptureMode(cudaStreamCaptureMode* m) {
+  const cudaStreamCaptureMode old = fake::mode;
+  fake::mode = *m;
+  *m = old;
+  return 0;
+}
+inline cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void*) { a->type = 0; return 0; }
+inline cudaError_t cudaMallocHost(void** p, size_t n) {
+  fake::Head* h = static_cast<fake::Head*>(std::malloc(sizeof(fake::Head) + n));
+  h->n = n;
+  *p = h + 1;
+  ++fake::pins;
+  fake::bytes += n;
+  return 0;
+}
+inline cudaError_t cudaFreeHost(void* p) {
+  fake::Head* h = static_cast<fake::Head*>(p) - 1;
+  fake::bytes -= h->n;
+  ++fake::frees;
+  std::free(h);
+  return 0;
+}
+inline cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, int) { ++fake::streams; *s = new Stream{fake::device}; return 0; }
+inline cudaError_t cudaStreamDestroy(cudaStream_t s) { ++fake::destroyed; delete s; return 0; }
+inline cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, int) { *e = new Event{fake::device}; return 0; }
+inline cudaError_t cudaEventDestroy(cudaEvent_t e) { delete e; return 0; }
+inline cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return 0; }
+inline cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, int) { return 0; }
+inline cudaError_t cudaStreamSynchronize(cudaStream_t) { ++fake::waits; return 0; }
+inline cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) {
+  std::memcpy(d, s, n);
+  ++fake::copies;
+  long long m = fake::piece;
+  while (m < (long long)n && !fake::piece.compare_exchange_weak(m, (long long)n)) {}
+  return 0;
+}
+'''
+
+SRC = r'''
+#include <new>
+#include "fgpu_transfer.h"
+using fgpu::Transfer;
+extern "C" {
+void* make() { return new Transfer; }
+void attach(void* t) { static_cast<Transfer*>(t)->attach(); }
+void detach(void* t) { static_cast<Transfer*>(t)->detach(); }
+int copy(void* t, void* host, void* dev, size_t n, int to_host, int device) {
+  return static_cast<Transfer*>(t)->copy(host, dev, n, to_host != 0, device, nullptr);
+}
+long long count(int what) {
+  std::atomic<long long>* c[] = {&fake::pins, &fake::frees, &fake::bytes, &fake::streams, &fake::destroyed,
+                                 &fake::copies, &fake::waits, &fake::piece};
+  return *c[what];
+}
+}
+'''
+PINS, FREES, PINNED, STREAMS, DESTROYED, COPIES, WAITS, PIECE = range(8)
+MB = 1 << 20
+
+
+@pytest.fixture(scope="module")
+def lib():
+    d = tempfile.mkdtemp()
+    for name, text in (("cuda_runtime.h", RUNTIME), ("t.cpp", SRC)):
+        with open(os.path.join(d, name), "w") as f:
+            f.write(text)
+    out = os.path.join(d, "libt.so")
+    subprocess.check_call([shutil.which("g++") or "g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-pthread", "-I", d, "-I", CSRC,
+                           "-o", out, os.path.join(d, "t.cpp")])
+    L = C.CDLL(out)
+    L.make.restype = C.c_void_p
+    L.count.restype = C.c_longlong
+    return L
+
+
+class _Lanes:
+    """A Transfer of its own, with the counts since it was made"""
+
+    def __init__(self, lib):
+        self.L, self.t = lib, C.c_void_p(lib.make())
+        self.start = [lib.count(q) for q in range(8)]
+
+    def count(self, what):
+        return self.L.count(what) - self.start[what]
+
+    def attach(self):
+        self.L.attach(self.t)
+
+    def detach(self):
+        self.L.detach(self.t)
+
+    def copy(self, n, to_host=True, device=0):
+        """Moves n bytes, each checked"""
+        src = np.frombuffer(np.random.default_rng(n).bytes(n), np.uint8)
+        dst = np.zeros(n, np.uint8)
+        host, dev = (dst, src) if to_host else (src, dst)
+        rc = self.L.copy(self.t, host.ctypes.data_as(C.c_void_p), dev.ctypes.data_as(C.c_void_p), C.c_size_t(n),
+                         C.c_int(to_host), C.c_int(device))
+        assert np.array_equal(src, dst)
+        return rc
+
+
+@pytest.mark.parametrize("n", [1 * MB, 1 * MB + 1, 3 * MB - 7, 9 * MB + 13, 70 * MB + 5])
+@pytest.mark.parametrize("to_host", [True, False])
+def test_every_byte_moves(lib, n, to_host):
+    t = _Lanes(lib)
+    t.attach()
+    assert t.copy(n, to_host) == 0
+    t.detach()
+
+
+def test_lanes_outlive_the_handles_that_use_them(lib):
+    """One grid after another, each closed before the next is opened: the slots are pinned once."""
+    t = _Lanes(lib)
+    for _ in range(5):
+        t.attach()
+        assert t.copy(2 * MB) == 0 and t.copy(MB + 64) == 0
+        t.detach()
+    assert t.count(PINS) == 1 and t.count(FREES) == 0 and t.count(STREAMS) <= 8
+
+
+def test_lanes_are_given_back(lib):
+    """A last handle that goes after no transfer used the lanes takes them along."""
+    t = _Lanes(lib)
+    t.attach()
+    t.copy(40 * MB)
+    t.detach()
+    assert t.count(PINNED) > 0
+    t.attach()
+    t.copy(MB // 2)
+    t.detach()
+    assert t.count(PINNED) == 0 and t.count(STREAMS) == t.count(DESTROYED)
+    t.attach()
+    assert t.copy(2 * MB) == 0
+    t.detach()
+
+
+def test_slots_grow_with_the_transfers(lib):
+    """Small grids pin little: a slot holds what has been asked of it, 4 MiB at most."""
+    t = _Lanes(lib)
+    t.attach()
+    t.copy(2 * MB)
+    lanes = t.count(STREAMS)
+    assert t.count(PINNED) == lanes * MB // 4
+    t.copy(200 * MB)
+    assert t.count(PINNED) == lanes * 4 * MB and t.count(PINS) == 2
+    t.copy(2 * MB)
+    assert t.count(PINNED) == lanes * 4 * MB and t.count(PINS) == 2
+    t.detach()
