@@ -9,10 +9,12 @@
 // cost (2 MiB in all 2 ms, 32 MiB 18 ms; freeing them 4 ms), so a slot holds the pieces asked
 // of it so far (256 KiB for transfers up to 4 MiB, 4 MiB from 64 MiB), and the lanes outlive the
 // handles: a program that opens, reads and closes one grid after another keeps them (freed with every
-// last handle they cost 35 ms a 256^2 grid).  They are given back when the last handle goes and no
-// transfer has used them since the previous time that it went; at most 32 MiB and eight streams stay.
+// last handle they cost 35 ms a 256^2 grid).  The slots serve every device, each of which has its own
+// streams, so that handles on two devices transfer in turn as those of one.  The lanes are given back
+// when the last handle goes and no transfer has used them since the previous time that it went; at
+// most 32 MiB and eight streams a device stay.
 // Transfers below kSmallDown / kSmallUp, pinned host memory, and calls that find the lanes in use or
-// cannot make them take the driver's path.  Thresholds (16 host cores, driver / lanes): downloads
+// cannot make them (devices past the kDevices-th too) take the driver's path.  Thresholds (16 host cores, driver / lanes): downloads
 // into fresh pages 0.5 MB 0.25 / 0.22 ms, 1.1 MB 0.54 / 0.21, 8.3 MB 4.0 / 1.0, 110 MB 52 / 9.5; uploads, whose
 // pages exist already, 4.2 MB 0.24 / 0.29 ms, 8.3 MB 0.46 / 0.43, 34 MB 3.0 / 1.2.
 #pragma once
@@ -29,7 +31,7 @@ class Transfer {
  public:
   static constexpr size_t kPiece = size_t(4) << 20, kLeast = size_t(256) << 10;
   static constexpr size_t kSmallDown = size_t(1) << 20, kSmallUp = size_t(8) << 20;
-  static constexpr int kLanes = 8;
+  static constexpr int kLanes = 8, kDevices = 16;
 
   static Transfer& shared() {
     static Transfer* t = new Transfer;   // (never destroyed: no CUDA calls at process exit)
@@ -53,31 +55,33 @@ class Transfer {
     std::unique_lock<std::mutex> lock(mutex_, std::defer_lock);
     if (bytes >= (to_host ? kSmallDown : kSmallUp) && !pinned(host)) (void)lock.try_lock();
     const OnDevice on(lock.owns_lock() ? device : -1);
-    if (!lock.owns_lock() || !prepare(device, bytes)) {
+    Device* const D = lock.owns_lock() ? prepare(device, bytes) : nullptr;
+    if (!D) {
       cudaError_t e = cudaMemcpyAsync(to_host ? host : dev, to_host ? dev : host, bytes, kind, s);
       return e != cudaSuccess ? e : cudaStreamSynchronize(s);
     }
     used_ = true;
-    cudaError_t e = cudaEventRecord(ready_, s);   // the lanes start after the work enqueued on s
+    cudaError_t e = cudaEventRecord(D->ready, s);   // the lanes start after the work enqueued on s
     if (e != cudaSuccess) return e;
-    const size_t piece = std::min(slot_bytes_, piece_bytes(bytes, lanes_.size()));
+    const size_t piece = std::min(slot_bytes_, piece_bytes(bytes, D->lanes));
     const size_t pieces = (bytes + piece - 1) / piece;
-    const int n = (int)std::min<size_t>(lanes_.size(), pieces);
+    const int n = (int)std::min<size_t>(D->lanes, pieces);
     std::vector<cudaError_t> err(n, cudaSuccess);
     const cudaStreamCaptureMode capture = capture_mode();
     auto work = [&](int t) {
-      Lane& L = lanes_[t];
+      const cudaStream_t stream = D->stream[t];
+      char* const slot = slots_ + t * slot_bytes_;
       cudaStreamCaptureMode mode = capture;   // the lane's threads wait under the caller's rules
       cudaError_t r = cudaThreadExchangeStreamCaptureMode(&mode);
       if (r == cudaSuccess) r = cudaSetDevice(device);
-      if (r == cudaSuccess) r = cudaStreamWaitEvent(L.stream, ready_, 0);
+      if (r == cudaSuccess) r = cudaStreamWaitEvent(stream, D->ready, 0);
       for (size_t p = t; p < pieces && r == cudaSuccess; p += n) {
         const size_t o = p * piece, m = std::min(piece, bytes - o);
         char *h = static_cast<char*>(host) + o, *d = static_cast<char*>(dev) + o;
-        if (!to_host) std::memcpy(L.slot, h, m);
-        r = cudaMemcpyAsync(to_host ? L.slot : d, to_host ? d : L.slot, m, kind, L.stream);
-        if (r == cudaSuccess) r = cudaStreamSynchronize(L.stream);
-        if (r == cudaSuccess && to_host) std::memcpy(h, L.slot, m);
+        if (!to_host) std::memcpy(slot, h, m);
+        r = cudaMemcpyAsync(to_host ? slot : d, to_host ? d : slot, m, kind, stream);
+        if (r == cudaSuccess) r = cudaStreamSynchronize(stream);
+        if (r == cudaSuccess && to_host) std::memcpy(h, slot, m);
       }
       err[t] = r;
     };
@@ -97,7 +101,11 @@ class Transfer {
   }
 
  private:
-  struct Lane { char* slot; cudaStream_t stream; };
+  struct Device {
+    int id = -1, lanes = 0;
+    cudaStream_t stream[kLanes] = {};
+    cudaEvent_t ready = nullptr;
+  };
   // two pieces a lane or more
   static size_t piece_bytes(size_t bytes, size_t lanes) {
     return std::min(kPiece, std::max(kLeast, (bytes / (2 * lanes) + 4095) / 4096 * 4096));
@@ -112,11 +120,9 @@ class Transfer {
     }
   };
   std::mutex mutex_;
-  std::vector<Lane> lanes_;
-  cudaEvent_t ready_ = nullptr;
+  Device devices_[kDevices];   // those with lanes first
   char* slots_ = nullptr;      // one pinned block, kLanes slots of slot_bytes_
   size_t slot_bytes_ = 0;
-  int device_ = -1;
   long long handles_ = 0;
   bool used_ = false;          // since the last handle last went
 
@@ -138,44 +144,46 @@ class Transfer {
     cudaThreadExchangeStreamCaptureMode(&mode);
     return callers;
   }
-  // lanes on this device (the last device's are given back first) with slots for pieces of a transfer
-  // of `bytes`, or smaller slots where no larger ones are to be had
-  bool prepare(int device, size_t bytes) {
-    if (device_ != device || lanes_.empty()) {
-      release();
-      if (cudaEventCreateWithFlags(&ready_, cudaEventDisableTiming) != cudaSuccess) ready_ = nullptr;
-      device_ = device;
-      const int want = std::max(1, std::min<int>(kLanes, (int)std::thread::hardware_concurrency() / 2));
-      for (int t = 0; t < want && ready_; ++t) {
-        Lane L = {nullptr, nullptr};
-        if (cudaStreamCreateWithFlags(&L.stream, cudaStreamNonBlocking) != cudaSuccess) break;
-        lanes_.push_back(L);
-      }
+  static int lane_count() { return std::max(1, std::min<int>(kLanes, (int)std::thread::hardware_concurrency() / 2)); }
+  // the lanes of the current device with slots for pieces of a transfer of `bytes`, or smaller
+  // slots where no larger ones are to be had
+  Device* prepare(int device, size_t bytes) {
+    Device* D = devices_;
+    while (D < devices_ + kDevices && D->id >= 0 && D->id != device) ++D;
+    if (D == devices_ + kDevices) return nullptr;
+    if (D->id < 0) {
+      if (cudaEventCreateWithFlags(&D->ready, cudaEventDisableTiming) != cudaSuccess) D->ready = nullptr;
+      while (D->ready && D->lanes < lane_count() &&
+             cudaStreamCreateWithFlags(&D->stream[D->lanes], cudaStreamNonBlocking) == cudaSuccess)
+        ++D->lanes;
+      if (D->lanes) D->id = device;
+      else release(*D);
     }
-    if (!lanes_.empty()) reserve(piece_bytes(bytes, lanes_.size()));
+    if (D->lanes) reserve(piece_bytes(bytes, D->lanes));
     cudaGetLastError();
-    if (lanes_.empty() || !slots_) release();
-    return slots_ != nullptr;
+    return D->lanes && slots_ ? D : nullptr;
   }
   void reserve(size_t piece) {
     size_t want = kLeast;
     while (want < piece) want *= 2;
     char* block = nullptr;
-    if (want <= slot_bytes_ || cudaMallocHost(reinterpret_cast<void**>(&block), want * lanes_.size()) != cudaSuccess) return;
+    if (want <= slot_bytes_ ||
+        cudaHostAlloc(reinterpret_cast<void**>(&block), want * lane_count(), cudaHostAllocPortable) != cudaSuccess)
+      return;
     if (slots_) cudaFreeHost(slots_);
     slots_ = block;
     slot_bytes_ = want;
-    for (size_t t = 0; t < lanes_.size(); ++t) lanes_[t].slot = slots_ + t * want;
+  }
+  static void release(Device& D) {
+    for (int t = 0; t < D.lanes; ++t) cudaStreamDestroy(D.stream[t]);
+    if (D.ready) cudaEventDestroy(D.ready);
+    D = Device();
   }
   void release() {
-    for (Lane& L : lanes_) cudaStreamDestroy(L.stream);
-    lanes_.clear();
+    for (Device& D : devices_) release(D);
     if (slots_) cudaFreeHost(slots_);
     slots_ = nullptr;
     slot_bytes_ = 0;
-    if (ready_) cudaEventDestroy(ready_);
-    ready_ = nullptr;
-    device_ = -1;
   }
 };
 

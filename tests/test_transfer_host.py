@@ -20,7 +20,7 @@ RUNTIME = r'''
 typedef int cudaError_t;
 typedef struct Stream { int device; } *cudaStream_t;
 typedef struct Event { int device; } *cudaEvent_t;
-enum { cudaSuccess = 0, cudaErrorMemoryAllocation = 2 };
+enum { cudaSuccess = 0, cudaErrorMemoryAllocation = 2, cudaErrorInvalidResourceHandle = 400 };
 enum { cudaStreamNonBlocking = 1, cudaEventDisableTiming = 2, cudaMemoryTypeUnregistered = 0 };
 enum cudaMemcpyKind { cudaMemcpyHostToDevice = 1, cudaMemcpyDeviceToHost = 2 };
 enum cudaStreamCaptureMode { cudaStreamCaptureModeGlobal, cudaStreamCaptureModeThreadLocal, cudaStreamCaptureModeRelaxed };
@@ -42,6 +42,7 @@ inline cudaError_t cudaThreadExchangeStreamCaptureMode(cudaStreamCaptureMode* m)
   return 0;
 }
 inline cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void*) { a->type = 0; return 0; }
+enum { cudaHostAllocPortable = 1 };
 inline cudaError_t cudaMallocHost(void** p, size_t n) {
   fake::Head* h = static_cast<fake::Head*>(std::malloc(sizeof(fake::Head) + n));
   h->n = n;
@@ -50,6 +51,7 @@ inline cudaError_t cudaMallocHost(void** p, size_t n) {
   fake::bytes += n;
   return 0;
 }
+inline cudaError_t cudaHostAlloc(void** p, size_t n, int) { return cudaMallocHost(p, n); }
 inline cudaError_t cudaFreeHost(void* p) {
   fake::Head* h = static_cast<fake::Head*>(p) - 1;
   fake::bytes -= h->n;
@@ -64,7 +66,8 @@ inline cudaError_t cudaEventDestroy(cudaEvent_t e) { delete e; return 0; }
 inline cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return 0; }
 inline cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, int) { return 0; }
 inline cudaError_t cudaStreamSynchronize(cudaStream_t) { ++fake::waits; return 0; }
-inline cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) {
+inline cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t stream) {
+  if (stream && stream->device != fake::device) return cudaErrorInvalidResourceHandle;
   std::memcpy(d, s, n);
   ++fake::copies;
   long long m = fake::piece;
@@ -183,4 +186,20 @@ def test_slots_grow_with_the_transfers(lib):
     assert t.count(PINNED) == lanes * 4 * MB and t.count(PINS) == 2
     t.copy(2 * MB)
     assert t.count(PINNED) == lanes * 4 * MB and t.count(PINS) == 2
+    t.detach()
+
+
+def test_devices_in_turn(lib):
+    """Handles on several devices that transfer in turn: the slots are pinned once, the streams of each
+    device made once, and every piece goes through a stream of its device."""
+    t = _Lanes(lib)
+    t.attach()
+    t.copy(2 * MB, device=0)
+    lanes = t.count(STREAMS)
+    for device in (0, 1, 2, 1, 0, 2):
+        assert t.copy(2 * MB, device=device) == 0
+    assert t.count(PINS) == 1 and t.count(STREAMS) == 3 * lanes and t.count(DESTROYED) == 0
+    for device in range(3, 20):   # more devices than have room: the driver's path
+        assert t.copy(2 * MB, device=device) == 0
+    assert t.count(STREAMS) <= 16 * lanes
     t.detach()
