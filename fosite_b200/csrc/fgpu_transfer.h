@@ -20,6 +20,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <mutex>
 #include <thread>
@@ -37,14 +38,13 @@ class Transfer {
     static Transfer* t = new Transfer;   // (never destroyed: no CUDA calls at process exit)
     return *t;
   }
-  // handles alive
-  void attach() {
-    std::lock_guard<std::mutex> lock(mutex_);
-    ++handles_;
-  }
+  // Handles alive.  Neither waits for a transfer: one in flight belongs to a handle that is alive, so
+  // that the lanes are not due.
+  void attach() { ++handles_; }
   void detach() {
-    std::lock_guard<std::mutex> lock(mutex_);
     if (--handles_ != 0) return;
+    std::unique_lock<std::mutex> lock(mutex_, std::try_to_lock);
+    if (!lock.owns_lock() || handles_ != 0) return;
     if (!used_) release();
     used_ = false;
   }
@@ -123,7 +123,7 @@ class Transfer {
   Device devices_[kDevices];   // those with lanes first
   char* slots_ = nullptr;      // one pinned block, kLanes slots of slot_bytes_
   size_t slot_bytes_ = 0;
-  long long handles_ = 0;
+  std::atomic<long long> handles_{0};
   bool used_ = false;          // since the last handle last went
 
   static bool pinned(const void* p) {

@@ -5,6 +5,8 @@ import os
 import shutil
 import subprocess
 import tempfile
+import threading
+import time
 
 import numpy as np
 import pytest
@@ -17,6 +19,7 @@ RUNTIME = r'''
 #include <atomic>
 #include <cstdlib>
 #include <cstring>
+#include <thread>
 typedef int cudaError_t;
 typedef struct Stream { int device; } *cudaStream_t;
 typedef struct Event { int device; } *cudaEvent_t;
@@ -28,6 +31,7 @@ struct cudaPointerAttributes { int type; };
 namespace fake {
 inline std::atomic<long long> pins{0}, frees{0}, bytes{0}, streams{0}, destroyed{0}, copies{0}, waits{0};
 inline std::atomic<long long> piece{0};   // of the largest copy
+inline std::atomic<int> held{0};          // copies wait while it is set
 inline thread_local int device = 0;
 inline thread_local cudaStreamCaptureMode mode = cudaStreamCaptureModeGlobal;
 struct Head { size_t n; char pad[56]; };
@@ -70,6 +74,7 @@ inline cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyK
   if (stream && stream->device != fake::device) return cudaErrorInvalidResourceHandle;
   std::memcpy(d, s, n);
   ++fake::copies;
+  while (fake::held) std::this_thread::yield();
   long long m = fake::piece;
   while (m < (long long)n && !fake::piece.compare_exchange_weak(m, (long long)n)) {}
   return 0;
@@ -87,6 +92,7 @@ void detach(void* t) { static_cast<Transfer*>(t)->detach(); }
 int copy(void* t, void* host, void* dev, size_t n, int to_host, int device) {
   return static_cast<Transfer*>(t)->copy(host, dev, n, to_host != 0, device, nullptr);
 }
+void hold(int on) { fake::held = on; }
 long long count(int what) {
   std::atomic<long long>* c[] = {&fake::pins, &fake::frees, &fake::bytes, &fake::streams, &fake::destroyed,
                                  &fake::copies, &fake::waits, &fake::piece};
@@ -202,4 +208,26 @@ def test_devices_in_turn(lib):
     for device in range(3, 20):   # more devices than have room: the driver's path
         assert t.copy(2 * MB, device=device) == 0
     assert t.count(STREAMS) <= 16 * lanes
+    t.detach()
+
+
+def test_handles_come_and_go_during_a_transfer(lib):
+    """Creating and closing a handle does not wait for another thread's transfer."""
+    t = _Lanes(lib)
+    t.attach()
+    lib.hold(1)
+    rc, done = [], threading.Event()
+    mover = threading.Thread(target=lambda: rc.append(t.copy(3 * MB)))
+    other = threading.Thread(target=lambda: (t.attach(), t.detach(), done.set()))
+    try:
+        mover.start()
+        while t.count(COPIES) == 0:
+            time.sleep(0.001)
+        other.start()
+        assert done.wait(20)
+    finally:
+        lib.hold(0)
+        mover.join()
+        other.join()
+    assert rc == [0]
     t.detach()
