@@ -24,7 +24,6 @@
 #include <cstring>
 #include <mutex>
 #include <thread>
-#include <vector>
 
 namespace fgpu {
 
@@ -49,7 +48,8 @@ class Transfer {
     used_ = false;
   }
   // bytes between device memory (ready in stream order of s) and host memory; returns when the copy
-  // is complete.  to_host: device to host, else host to device (later work of s sees it).
+  // is complete.  to_host: device to host, else host to device (later work of s sees it).  Its callers are
+  // C entries: nothing here throws.
   cudaError_t copy(void* host, void* dev, size_t bytes, bool to_host, int device, cudaStream_t s) {
     const cudaMemcpyKind kind = to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice;
     std::unique_lock<std::mutex> lock(mutex_, std::defer_lock);
@@ -66,7 +66,7 @@ class Transfer {
     const size_t piece = std::min(slot_bytes_, piece_bytes(bytes, D->lanes));
     const size_t pieces = (bytes + piece - 1) / piece;
     const int n = (int)std::min<size_t>(D->lanes, pieces);
-    std::vector<cudaError_t> err(n, cudaSuccess);
+    cudaError_t err[kLanes] = {};
     const cudaStreamCaptureMode capture = capture_mode();
     auto work = [&](int t) {
       const cudaStream_t stream = D->stream[t];
@@ -85,16 +85,15 @@ class Transfer {
       }
       err[t] = r;
     };
-    std::vector<std::thread> threads;
-    threads.reserve(n);
+    std::thread threads[kLanes];
     int started = 1;
     try {
-      for (; started < n; ++started) threads.emplace_back(work, started);
-    } catch (...) {   // no more threads: this one takes the remaining lanes' pieces
+      for (; started < n; ++started) threads[started] = std::thread(work, started);
+    } catch (...) {   // no more threads (or no memory for them): this one takes the remaining lanes' pieces
     }
     work(0);
     for (int t = started; t < n; ++t) work(t);
-    for (auto& t : threads) t.join();
+    for (int t = 1; t < started; ++t) threads[t].join();
     for (cudaError_t r : err)
       if (r != cudaSuccess) return r;
     return cudaSuccess;

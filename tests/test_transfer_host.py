@@ -85,13 +85,26 @@ SRC = r'''
 #include <new>
 #include "fgpu_transfer.h"
 using fgpu::Transfer;
+static std::atomic<int> starved{0};
+void* operator new(size_t n) {
+  void* p = starved ? nullptr : std::malloc(n);
+  if (!p) throw std::bad_alloc();
+  return p;
+}
+void operator delete(void* p) noexcept { std::free(p); }
+void operator delete(void* p, size_t) noexcept { std::free(p); }
 extern "C" {
 void* make() { return new Transfer; }
 void attach(void* t) { static_cast<Transfer*>(t)->attach(); }
 void detach(void* t) { static_cast<Transfer*>(t)->detach(); }
 int copy(void* t, void* host, void* dev, size_t n, int to_host, int device) {
-  return static_cast<Transfer*>(t)->copy(host, dev, n, to_host != 0, device, nullptr);
+  try {
+    return static_cast<Transfer*>(t)->copy(host, dev, n, to_host != 0, device, nullptr);
+  } catch (...) {
+    return -1;
+  }
 }
+void starve(int on) { starved = on; }
 void hold(int on) { fake::held = on; }
 long long count(int what) {
   std::atomic<long long>* c[] = {&fake::pins, &fake::frees, &fake::bytes, &fake::streams, &fake::destroyed,
@@ -111,7 +124,7 @@ def lib():
         with open(os.path.join(d, name), "w") as f:
             f.write(text)
     out = os.path.join(d, "libt.so")
-    subprocess.check_call([shutil.which("g++") or "g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-pthread", "-I", d, "-I", CSRC,
+    subprocess.check_call([shutil.which("g++") or "g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-pthread", "-Wl,-Bsymbolic", "-I", d, "-I", CSRC,
                            "-o", out, os.path.join(d, "t.cpp")])
     L = C.CDLL(out)
     L.make.restype = C.c_void_p
@@ -230,4 +243,19 @@ def test_handles_come_and_go_during_a_transfer(lib):
         mover.join()
         other.join()
     assert rc == [0]
+    t.detach()
+
+
+@pytest.mark.parametrize("to_host", [True, False])
+def test_no_memory_for_threads(lib, to_host):
+    """A transfer that can start no threads moves every piece itself; no exception reaches the C entry."""
+    t = _Lanes(lib)
+    t.attach()
+    assert t.copy(9 * MB, to_host) == 0
+    lib.starve(1)
+    try:
+        rc = t.copy(9 * MB, to_host)
+    finally:
+        lib.starve(0)
+    assert rc == 0
     t.detach()
