@@ -47,9 +47,9 @@ class Transfer {
     if (!used_) release();
     used_ = false;
   }
-  // bytes between device memory (ready in stream order of s) and host memory; returns when the copy
-  // is complete.  to_host: device to host, else host to device (later work of s sees it).  Its callers are
-  // C entries: nothing here throws.
+  // bytes between device memory (ready in stream order of s) and host memory.  to_host: device to
+  // host, complete on return; else host to device: later work of s sees it, and the host array is
+  // read until s has been waited for.  Its callers are C entries: nothing here throws.
   cudaError_t copy(void* host, void* dev, size_t bytes, bool to_host, int device, cudaStream_t s) {
     const cudaMemcpyKind kind = to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice;
     std::unique_lock<std::mutex> lock(mutex_, std::defer_lock);
@@ -58,7 +58,7 @@ class Transfer {
     Device* const D = lock.owns_lock() ? prepare(device, bytes) : nullptr;
     if (!D) {
       cudaError_t e = cudaMemcpyAsync(to_host ? host : dev, to_host ? dev : host, bytes, kind, s);
-      return e != cudaSuccess ? e : cudaStreamSynchronize(s);
+      return e != cudaSuccess || !to_host ? e : cudaStreamSynchronize(s);
     }
     used_ = true;
     cudaError_t e = cudaEventRecord(D->ready, s);   // the lanes start after the work enqueued on s

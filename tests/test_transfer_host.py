@@ -259,3 +259,13 @@ def test_no_memory_for_threads(lib, to_host):
         lib.starve(0)
     assert rc == 0
     t.detach()
+
+
+def test_small_uploads_are_enqueued(lib):
+    """A small upload does not wait for its stream (its caller does, after the kernel that unpacks it); a
+    download does."""
+    t = _Lanes(lib)
+    t.attach()
+    assert t.copy(4096, to_host=False) == 0 and t.count(WAITS) == 0
+    assert t.copy(4096, to_host=True) == 0 and t.count(WAITS) == 1
+    t.detach()
