@@ -830,12 +830,14 @@ int fgpu_batch_autotune(fgpu_batch* b, int reps, int* variant) {
 }  // extern "C"
 
 namespace {
-// Tuning decisions of this process, by the key of what the stage kernel's cost depends on
-// (device, dimensionality, physics, reconstruction variables and limiter, geometry, mesh
-// size and the optional source/transport features): a grid with a known key reuses the
-// measured layout without probing.
+// Tuning decisions of this process, by the key of what decides which kernel the probe runs and
+// what its cost depends on: device, dimensionality, physics, reconstruction variables and order, the
+// compiled-in limiter (MC with theta = 1 is minmod code) and the limiter itself, the scheme (time order,
+// stages, formed states), geometry, boundaries (element copies at periodic faces, exp and log at
+// absorbing ones), mesh size and the optional source and transport features with the transport's direction.  A grid with a known
+// key reuses the measured layout without probing.
 struct TuneKey {
-  int device, nd, euler, prim, order, limiter, geometry, nx, ny, nz, features;
+  int device, nd, euler, prim, order, limiter, compiled, torder, stages, geometry, nx, ny, nz, bc[6], features;
   bool operator<(const TuneKey& o) const {
     return std::memcmp(this, &o, sizeof(TuneKey)) < 0;
   }
@@ -848,9 +850,14 @@ TuneKey tune_key(const fgpu_handle* h) {
   std::memset(&k, 0, sizeof(k));
   k.device = h->device; k.nd = h->nd; k.euler = h->euler; k.prim = h->prim;
   k.order = h->cfg.order; k.limiter = h->cfg.limiter; k.geometry = h->cfg.geometry;
+  k.compiled = compiled_limiter(h->cfg.limiter, h->cfg.order == FGPU_CONSTANT, h->cfg.theta);
+  k.torder = h->order;
+  k.stages = h->butcher ? h->T.m : 0;
+  for (int f = 0; f < 2 * h->nd; ++f) k.bc[f] = h->g.bc[f];
   k.nx = h->g.nx; k.ny = h->g.ny; k.nz = h->g.nz;
   k.features = (h->fargo ? 1 : 0) | (h->accrete ? 2 : 0) | (h->vis ? 4 : 0) | (h->has_accel ? 8 : 0) |
-               (h->butcher ? 16 : 0) | (h->materialize ? 32 : 0);
+               (h->butcher ? 16 : 0) | (h->materialize ? 32 : 0) | (h->fuse_form ? 64 : 0) | (h->so_form ? 128 : 0) |
+               (h->adaptive_me ? 256 : 0) | h->fdir << 10;
   return k;
 }
 }  // namespace

@@ -276,8 +276,8 @@ int fgpu_set_output_time(fgpu_handle* h, double tout);
 /* Measure every stage-kernel layout on this grid (reps RHS evaluations each into
  * a scratch array; the state is untouched) and keep the fastest for later
  * steps.  *variant receives the choice.  Decisions are cached per process by
- * (device, dimensionality, physics, reconstruction variables, limiter, geometry,
- * mesh size, features): a grid with a known key takes the cached layout without
+ * (device, dimensionality, physics, reconstruction variables, limiter, time scheme, geometry,
+ * boundaries, mesh size, features): a grid with a known key takes the cached layout without
  * probing; reps < 0 measures |reps| times anyway and refreshes the entry.  No
  * counterpart in the reference. */
 int fgpu_autotune(fgpu_handle* h, int reps, int* variant);

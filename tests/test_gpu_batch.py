@@ -399,3 +399,40 @@ def test_adaptive_modified_euler_batch_equals_lone_runs(order):
     assert o.status().time == members[1].status().time
     assert np.array_equal(o.get(abi.CVAR), members[1].get(abi.CVAR))
     b.close()
+
+
+_TUNE_BASE = dict(method=abi.MODIFIED_EULER, tdorder=3, limiter=abi.MONOCENT, theta=1.0)
+_TUNE_OTHER = {"theta": dict(theta=1.2), "time_order": dict(tdorder=2),
+               "stages": dict(method=abi.CASH_KARP, tdorder=5), "boundaries": dict(bcs=[abi.PERIODIC] * 6)}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("other", list(_TUNE_OTHER))
+def test_tuner_cache_tells_kernels_apart(other, monkeypatch):
+    """A cached choice serves grids whose stage runs the kernel that was timed: not one of another
+    compiled limiter (MC with theta 1 is minmod code), another number of stages or other boundaries.
+    The entry is recognised by its z chunk, 5, which the tuner times only while FGPU_KCHUNK is 5."""
+    from fosite_b200.sim import Simulation
+    from cases import _gauss3d
+
+    def chunk(forced, **kw):
+        kw = dict(_TUNE_BASE, **kw)
+        theta = kw.pop("theta")
+        cfg, p, _ = _gauss3d(n=(26, 22, 18), **kw)
+        cfg.theta = theta
+        if forced:
+            monkeypatch.setenv("FGPU_KCHUNK", "5")
+        else:
+            monkeypatch.delenv("FGPU_KCHUNK", raising=False)
+        s = Simulation(cfg)
+        assert forced or s.stage_layout()[1] != 5
+        s.set_state(abi.PVAR, p)
+        s.autotune(-1 if forced else 1)
+        k = s.stage_layout()[1]
+        s.close()
+        return k
+
+    start = dict(method=abi.DORMAND_PRINCE, tdorder=5) if other == "stages" else {}
+    assert chunk(True, **start) == 5
+    assert chunk(False, **start) == 5
+    assert chunk(False, **_TUNE_OTHER[other]) != 5
