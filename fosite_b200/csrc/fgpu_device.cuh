@@ -187,9 +187,10 @@ __device__ __forceinline__ double dmax(double a, double b) { return fmax(a, b); 
 // (1/d: y + y (e + e^2) with e = 1 - d y; 1/sqrt(q): y + y (e/2 + 3 e^2/8) with e = 1 - q y^2),
 // which cubes the relative error.  Straight-line code: the compiler's division and square root
 // carry a branch to a slow path at every use, and the stage kernels hold up to twenty of them.
-// d and q must be normal, finite and not within a factor 2^2 of the range's ends (in_range);
-// 0, infinities and NaN give NaN.  Measured over 12.6 million values of exponents -950 to 950 the
-// largest relative errors are 1.00 (reciprocal) and 1.25 (square root) times 2^-53; with the
+// d and its reciprocal must be normal (2^-1022 <= |d| < 2^1022; DBL_MIN, the smallest denominator of
+// the van Leer slope, gives 2^1022 exactly), q normal.  0, infinities, NaN and a subnormal d give NaN, a
+// subnormal q an infinity.  The relative errors are at most 1.00 (the closing addition's rounding) and
+// 1.5 (with that of q y, halved) times 2^-53, checked over those ranges (test_gpu_refined.py); with the
 // selections of the limiters and wave speeds below the 256^3 Dormand-Prince step went from
 // 17.0 to 14.2 ms, the 2D boxes' steps by 4 to 11%.
 __device__ __forceinline__ double rcp_refined(double d) {
@@ -260,7 +261,7 @@ struct Phys {
   // GetSoundSpeed (physics_euler.f90:2682-2689): sqrt(MAX(2 TINY, gamma*p/rho)).
   // The product build evaluates sqrt(s/rho) as s*rsqrt(s*rho) with s = gamma*p (within a few
   // ulp).  Wherever s*rho leaves the normal range, or s or rho is not positive, that form gives
-  // a NaN, a negative value or one below the floor sqrt(2 TINY) = 2^-510.5 (cs_good); the
+  // a NaN, an infinity, a negative value or one below the floor sqrt(2 TINY) = 2^-510.5 (cs_good); the
   // reference's form then takes over.
   static __device__ __forceinline__ double cs_of(const double* p, const PhysP& P) {
 #ifdef FGPU_EXACT

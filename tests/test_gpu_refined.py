@@ -1,0 +1,80 @@
+"""The refined reciprocal and reciprocal square root of the product build (fgpu_device.cuh) against
+their error bounds, over the ends of the range that the stage kernels use them in: the source is compiled
+into a small probe and its results compared in 64-bit mantissas (x87)."""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from fosite_b200 import build
+
+SRC = r'''
+#include "fgpu_device.cuh"
+__global__ void probe(const double* x, double* y, int n, int root) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) y[i] = root ? fgpu::rsqrt_refined(x[i]) : fgpu::rcp_refined(x[i]);
+}
+extern "C" int run(const double* x, double* y, int n, int root) {
+  double* d;
+  if (cudaMalloc(&d, 2 * sizeof(double) * n) != cudaSuccess) return 1;
+  cudaMemcpy(d, x, sizeof(double) * n, cudaMemcpyHostToDevice);
+  probe<<<(n + 255) / 256, 256>>>(d, d + n, n, root);
+  const cudaError_t e = cudaMemcpy(y, d + n, sizeof(double) * n, cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  return e != cudaSuccess;
+}
+'''
+
+
+@pytest.fixture(scope="module")
+def probe(tmp_path_factory):
+    d = tmp_path_factory.mktemp("refined")
+    src, out = str(d / "probe.cu"), str(d / "probe.so")
+    with open(src, "w") as f:
+        f.write(SRC)
+    subprocess.check_call([build.nvcc(), "-O3", "-std=c++17", "--expt-relaxed-constexpr", *build.ARCH, "-shared", "-Xcompiler",
+                           "-fPIC", "-I", build.CSRC, "-I", os.path.join(build.HERE, "..", "include"), "-o", out, src])
+    run = C.CDLL(out).run
+
+    def call(x, root):
+        y = np.empty_like(x)
+        assert run(x.ctypes.data_as(C.c_void_p), y.ctypes.data_as(C.c_void_p), C.c_int(x.size), C.c_int(root)) == 0
+        return y
+    return call
+
+
+def _values(lo, hi, n=4_000_000):
+    """Mantissas over [1, 2) at exponents lo .. hi - 1, with the ends and neighbours of the powers of two"""
+    rng = np.random.default_rng(17)
+    x = np.ldexp(rng.uniform(1.0, 2.0, n), rng.integers(lo, hi, n))
+    p = np.ldexp(1.0, np.arange(lo, hi))
+    return np.concatenate([x, p, np.nextafter(p, np.inf), np.ldexp(np.nextafter(2.0, 0.0), np.arange(lo, hi))])
+
+
+@pytest.mark.gpu
+def test_reciprocal(probe):
+    """1/d for every normal d whose reciprocal is normal, of either sign, DBL_MIN among them (the van Leer
+    slope's smallest denominator).  The cubed error of the approximation stays below 2^-60 and 1 - d y is
+    rounded in a term 2^-20 of the result, so that the closing addition's half ulp, at most 2^-53, is the error."""
+    d = _values(-1022, 1022)
+    d = np.concatenate([d, -d])
+    y = probe(d, 0)
+    err = np.abs(y.astype(np.longdouble) * d.astype(np.longdouble) - 1)
+    assert np.isfinite(y).all() and float(err.max()) <= 2.0 ** -53 * (1 + 2.0 ** -10)
+    assert probe(np.array([2.0 ** -1022]), 0)[0] == 2.0 ** 1022
+    assert np.isnan(probe(np.array([0.0, np.inf, -np.inf, np.nan, 5e-324, -2.0 ** -1023]), 0)).all()
+
+
+@pytest.mark.gpu
+def test_reciprocal_square_root(probe):
+    """1/sqrt(q) for every normal q: q y is rounded, at most 2^-53 of it, which the correction halves; the
+    closing addition's half ulp comes on top: at most 1.5 x 2^-53."""
+    q = _values(-1022, 1024)
+    y = probe(q, 1)
+    y80 = y.astype(np.longdouble)
+    err = np.abs(y80 * y80 * q.astype(np.longdouble) - 1) / 2
+    assert np.isfinite(y).all() and float(err.max()) <= 1.5 * 2.0 ** -53 * (1 + 2.0 ** -10)
+    assert np.isnan(probe(np.array([0.0, np.inf, -1.0, np.nan]), 1)).all()
+    assert not np.isfinite(probe(np.array([5e-324, 2.0 ** -1023]), 1)).any()   # an infinite sound speed is not good
