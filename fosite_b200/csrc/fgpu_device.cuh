@@ -205,6 +205,11 @@ __device__ __forceinline__ double rsqrt_refined(double q) {
   const double e = fma(-q * y, y, 1.0);
   return fma(y * e, fma(0.375, e, 0.5), y);
 }
+// 1/d of a cell width: a ghost cell whose centre lies on the axis has none along the angle, and its
+// quotients are infinite (a time step of 0) or, 0/0, NaN
+__device__ __forceinline__ double rcp_width(double d) {
+  return d == 0.0 ? copysign(__longlong_as_double(0x7ff0000000000000LL), d) : rcp_refined(d);
+}
 // 2^-LO <= x < 2^HI (x positive), by its exponent: one integer subtraction and comparison
 template <int LO, int HI>
 __device__ __forceinline__ bool in_range(double x) {
@@ -598,7 +603,7 @@ struct Cells {
 #ifdef FGPU_EXACT
       a[m] = w[m] / dl[m];
 #else
-      a[m] = w[m] * rcp_refined(dl[m]);
+      a[m] = w[m] * rcp_width(dl[m]);
 #endif
     }
     if (ND == 2) { out[0] = a[0] + a[1]; out[1] = 0.0; out[2] = 0.0; }

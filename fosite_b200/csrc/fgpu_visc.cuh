@@ -119,7 +119,7 @@ __device__ __forceinline__ double width_inverse(double d) {
 #ifdef FGPU_EXACT
   return d;
 #else
-  return rcp_refined(d);
+  return rcp_width(d);
 #endif
 }
 __device__ __forceinline__ double over(double x, double d, double rd) {

@@ -8,7 +8,8 @@ import subprocess
 import numpy as np
 import pytest
 
-from fosite_b200 import build
+from fosite_b200 import abi, build
+from cases import _visc
 
 SRC = r'''
 #include "fgpu_device.cuh"
@@ -78,3 +79,57 @@ def test_reciprocal_square_root(probe):
     assert np.isfinite(y).all() and float(err.max()) <= 1.5 * 2.0 ** -53 * (1 + 2.0 ** -10)
     assert np.isnan(probe(np.array([0.0, np.inf, -1.0, np.nan]), 1)).all()
     assert not np.isfinite(probe(np.array([5e-324, 2.0 ** -1023]), 1)).any()   # an infinite sound speed is not good
+
+
+def _ring():
+    """A cylindrical mesh that starts half a cell from the axis: the centre of the first inner ghost
+    column lies on it, with no width along the angle."""
+    c = abi.default_config()
+    c.inum, c.jnum, c.knum = 16, 24, 1
+    c.geometry = abi.CYLINDRICAL
+    c.xmin, c.xmax, c.ymin, c.ymax = 0.03125, 1.03125, 0.0, 2 * np.pi
+    c.physics, c.gamma = abi.EULER, 1.4
+    c.limiter, c.variables = abi.VANLEER, abi.CONSERVATIVE
+    c.method, c.tdorder, c.tol_rel = abi.MODIFIED_EULER, 3, 10.0
+    c.cfl, c.stoptime = 0.4, 1.0e3
+    for f, t in enumerate((abi.NO_GRADIENTS, abi.NO_GRADIENTS, abi.PERIODIC, abi.PERIODIC)):
+        c.bc[f] = t
+    abi.finalize_config(c)
+    p = np.ones((4, 1, 28, 20))
+    p[1:3] = np.random.default_rng(0).uniform(-0.1, 0.1, (2, 1, 28, 20))
+    return c, p, {}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("exact", [True, False])
+def test_time_step_of_a_ghost_cell_without_width(exact):
+    """CalcTimestep's maximum runs over the ghost cells too: the oracle's step is 0 there."""
+    from fosite_b200.sim import Simulation
+    pyoracle = pytest.importorskip("pyoracle")
+    cfg, p, _ = _ring()
+    o, g = pyoracle.Oracle(cfg), Simulation(cfg, exact=exact)
+    for s in (o, g):
+        s.set_state(abi.PVAR, p)
+        s.first_step()
+    assert o.status().dt == 0.0 and g.status().dt == 0.0
+    assert g.calc_timestep() == 0.0
+    g.close()
+
+
+@pytest.mark.gpu
+def test_stresses_of_a_ghost_cell_without_width():
+    """Infinities and NaN of the viscous source are where the quotients of the exact build have them."""
+    from fosite_b200.sim import Simulation
+    cfg, p, _ = _visc(_ring(), 0.01)
+    rhs = []
+    for exact in (True, False):
+        g = Simulation(cfg, exact=exact)
+        g.set_state(abi.PVAR, p)
+        rhs.append(g.compute_rhs()[:, :, 2:-2, 2:-2])
+        g.close()
+    a, b = rhs
+    assert not np.isfinite(a).all()
+    for kind in (np.isnan, np.isposinf, np.isneginf):
+        assert np.array_equal(kind(a), kind(b))
+    m = np.isfinite(a)
+    assert np.abs(a[m] - b[m]).sum() <= 1e-12 * np.abs(a[m]).sum()
