@@ -1,24 +1,32 @@
 // fgpu_transfer.h -- copies between the device and a caller's pageable host arrays.
 //
 // cudaMemcpyAsync on pageable memory goes through one staging buffer of the driver on one host
-// core: 4.8 GB/s into fresh pages (703 MB of a 256^3 state: 150 ms, thirteen of its steps).  Here up
+// core: 2 to 5 GB/s into fresh pages (703 MB of a 256^3 state: 150 to 340 ms).  Here up
 // to kLanes host threads, each with its own pinned slot and stream, move interleaved pieces: one
 // piece is on the bus while others are copied between pinned and pageable memory (whose page faults
 // are what a core spends its time on).  The lanes are shared by all handles of the process, used by
 // one transfer at a time, and made at the first large transfer: pinning their slots is what they
 // cost (2 MiB in all 2 ms, 32 MiB 18 ms; freeing them 4 ms), so a slot holds the pieces asked
-// of it so far (256 KiB for transfers up to 4 MiB, 4 MiB from 64 MiB), and the lanes outlive the
+// of it so far (256 KiB for transfers up to 4 MiB, 4 MiB from 32 MiB on), and the lanes outlive the
 // handles: a program that opens, reads and closes one grid after another keeps them (freed with every
 // last handle they cost 35 ms a 256^2 grid).  The slots serve every device, each of which has its own
 // streams, so that handles on two devices transfer in turn as those of one.  The lanes are given back
 // when the last handle goes and no transfer has used them since the previous time that it went; at
 // most 32 MiB and eight streams a device stay.
-// Transfers below kSmallDown / kSmallUp, pinned host memory, and calls that find the lanes in use or
-// cannot make them (devices past the kDevices-th too) take the driver's path.  Thresholds (16 host cores, driver / lanes): downloads
-// into fresh pages 0.5 MB 0.25 / 0.22 ms, 1.1 MB 0.54 / 0.21, 8.3 MB 4.0 / 1.0, 110 MB 52 / 9.5; uploads, whose
-// pages exist already, 4.2 MB 0.24 / 0.29 ms, 8.3 MB 0.46 / 0.43, 34 MB 3.0 / 1.2.
+// Pinned host memory, transfers below the thresholds, and calls that find the lanes in use or cannot
+// make them (devices past the kDevices-th too) take the driver's path.  Thresholds, by what bounds
+// the driver's one core (16 host cores, ms, driver / lanes):
+//   * downloads into pages that do not exist yet, its page faults: 0.5 MB 0.25 / 0.22, 1.1 MB 0.54 / 0.21,
+//     8.3 MB 4.0 / 1.0, 110 MB 52 / 9.5;
+//   * downloads into resident pages (an allocator that reuses memory, or the caller's own array), its copy:
+//     2.2 MB 0.15 / 0.31, 5.5 MB 0.35 / 0.56, 12.6 MB 0.67 / 0.59 (one download after another; after
+//     another core's use 0.68 / 0.79, 34 MB 1.8 / 1.4); the lanes leave the array in their cores'
+//     caches, and its next reader pays for that (2.2 MB 0.11 / 0.32, 34 MB 1.7 / 2.0);
+//   * uploads: 4.2 MB 0.24 / 0.29, 8.3 MB 0.46 / 0.43, 34 MB 3.0 / 1.2.
 #pragma once
 #include <cuda_runtime.h>
+#include <sys/mman.h>
+#include <unistd.h>
 #include <algorithm>
 #include <atomic>
 #include <cstring>
@@ -30,7 +38,7 @@ namespace fgpu {
 class Transfer {
  public:
   static constexpr size_t kPiece = size_t(4) << 20, kLeast = size_t(256) << 10;
-  static constexpr size_t kSmallDown = size_t(1) << 20, kSmallUp = size_t(8) << 20;
+  static constexpr size_t kFreshDown = size_t(1) << 20, kDown = size_t(10) << 20, kUp = size_t(8) << 20;
   static constexpr int kLanes = 8, kDevices = 16;
 
   static Transfer& shared() {
@@ -53,7 +61,8 @@ class Transfer {
   cudaError_t copy(void* host, void* dev, size_t bytes, bool to_host, int device, cudaStream_t s) {
     const cudaMemcpyKind kind = to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice;
     std::unique_lock<std::mutex> lock(mutex_, std::defer_lock);
-    if (bytes >= (to_host ? kSmallDown : kSmallUp) && !pinned(host)) (void)lock.try_lock();
+    const bool lanes = !to_host ? bytes >= kUp : bytes >= kDown || (bytes >= kFreshDown && fresh(host, bytes));
+    if (lanes && !pinned(host)) (void)lock.try_lock();
     const OnDevice on(lock.owns_lock() ? device : -1);
     Device* const D = lock.owns_lock() ? prepare(device, bytes) : nullptr;
     if (!D) {
@@ -125,6 +134,17 @@ class Transfer {
   std::atomic<long long> handles_{0};
   bool used_ = false;          // since the last handle last went
 
+  // whether most of a host array's pages do not exist yet (sixteen of them are looked at)
+  static bool fresh(const void* host, size_t bytes) {
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE), first = reinterpret_cast<size_t>(host);
+    int absent = 0;
+    for (size_t q = 0; q < 16; ++q) {
+      unsigned char resident = 1;
+      const size_t at = (first + bytes / 32 * (2 * q + 1)) / page * page;
+      if (mincore(reinterpret_cast<void*>(at), page, &resident) == 0 && !(resident & 1)) ++absent;
+    }
+    return absent > 8;
+  }
   static bool pinned(const void* p) {
     cudaPointerAttributes a;
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {

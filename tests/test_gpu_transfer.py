@@ -22,8 +22,8 @@ def _interior(a, cfg):
     return a[:, 2:-2, 2:-2, 2:-2] if cfg.knum > 1 else a[:, :, 2:-2, 2:-2]
 
 
-# ghost-padded bytes: around 1 MiB (downloads take the lanes from there), 4.2 MB in odd rows, 48 and 110 MB
-# (uploads too, from 8 MiB)
+# ghost-padded bytes: around 1 MiB (downloads into fresh pages take the lanes from there), 4.2 MB in odd rows, 48 and
+# 110 MB (uploads too, from 8 MiB)
 @pytest.mark.gpu
 @pytest.mark.parametrize("case", [_khi(n=(36, 36)), _khi(n=(1021, 27)), _khi(n=(252, 125)), _khi(n=(509, 251)),
                                   _gauss3d(n=(100, 100, 106)), _gauss3d(n=(131, 133, 137))],

@@ -1,6 +1,7 @@
 """The pinned lanes of large transfers (fosite_b200/csrc/fgpu_transfer.h) on the host: the header compiled
 against a stand-in for the CUDA runtime that copies with memcpy and counts what it is asked for."""
 import ctypes as C
+import mmap
 import os
 import shutil
 import subprocess
@@ -148,10 +149,12 @@ class _Lanes:
     def detach(self):
         self.L.detach(self.t)
 
-    def copy(self, n, to_host=True, device=0):
-        """Moves n bytes, each checked"""
+    def copy(self, n, to_host=True, device=0, resident=False):
+        """Moves n bytes, each checked, into pages that do not exist yet or (resident) into existing ones"""
         src = np.frombuffer(np.random.default_rng(n).bytes(n), np.uint8)
-        dst = np.zeros(n, np.uint8)
+        dst = np.frombuffer(mmap.mmap(-1, n, flags=mmap.MAP_PRIVATE | mmap.MAP_ANONYMOUS), np.uint8)
+        if resident:
+            dst[:] = 0
         host, dev = (dst, src) if to_host else (src, dst)
         rc = self.L.copy(self.t, host.ctypes.data_as(C.c_void_p), dev.ctypes.data_as(C.c_void_p), C.c_size_t(n),
                          C.c_int(to_host), C.c_int(device))
@@ -268,4 +271,24 @@ def test_small_uploads_are_enqueued(lib):
     t.attach()
     assert t.copy(4096, to_host=False) == 0 and t.count(WAITS) == 0
     assert t.copy(4096, to_host=True) == 0 and t.count(WAITS) == 1
+    t.detach()
+
+
+@pytest.mark.parametrize("n,resident,lanes", [(MB - 8, False, False), (MB, False, True), (MB, True, False), (9 * MB, True, False),
+                                              (10 * MB, True, True), (10 * MB, False, True)])
+def test_downloads_by_their_pages(lib, n, resident, lanes):
+    """Lanes for pages that have to be made; one core's copy into pages that exist is as fast up to 10 MB."""
+    t = _Lanes(lib)
+    t.attach()
+    assert t.copy(n, resident=resident) == 0
+    assert (t.count(STREAMS) > 0) == lanes
+    t.detach()
+
+
+@pytest.mark.parametrize("n,lanes", [(8 * MB - 8, False), (8 * MB, True)])
+def test_uploads_by_their_size(lib, n, lanes):
+    t = _Lanes(lib)
+    t.attach()
+    assert t.copy(n, to_host=False) == 0
+    assert (t.count(STREAMS) > 0) == lanes
     t.detach()
