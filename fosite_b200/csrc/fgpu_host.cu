@@ -38,6 +38,13 @@ namespace {
 
 std::string g_create_error;
 
+// the lanes of the library's transfers (never destroyed: no CUDA calls at process exit); internal to the
+// library, so that two builds of it in one process do not share one object
+Transfer& transfers() {
+  static Transfer* t = new Transfer;
+  return *t;
+}
+
 struct Tableau {
   int m = 0, order = 0;
   std::vector<double> A, bh, bl, c;
@@ -1685,7 +1692,7 @@ int fgpu_create(const fgpu_config* cfg, int device, fgpu_handle** out) {
   if (!cfg || !out) return set_err(nullptr, FGPU_EARG, "null argument");
   *out = nullptr;
   fgpu_handle* h = new fgpu_handle();
-  Transfer::shared().attach();
+  transfers().attach();
   std::memset(&h->stats, 0, sizeof(h->stats));
   h->cfg = *cfg;
   int rc = validate(h);
@@ -1837,7 +1844,7 @@ void fgpu_destroy(fgpu_handle* h) {
   if (h->h_ctl) cudaFreeHost(h->h_ctl);
   if (h->own_stream) h->stream = h->own_stream;
   if (h->stream) cudaStreamDestroy(h->stream);
-  Transfer::shared().detach();
+  transfers().detach();
   delete h;
 }
 
@@ -1927,7 +1934,7 @@ int fgpu_upload_state(fgpu_handle* h, int which, const double* data, int64_t n) 
   if (which != FGPU_CVAR && which != FGPU_PVAR) return set_err(h, FGPU_EARG, "upload CVAR or PVAR");
   long long nc = fgpu_cell_count(h);
   if (!h->d_pad) CUDA_TRY(h, cudaMalloc(&h->d_pad, sizeof(double) * 2 * nc * h->V));
-  CUDA_TRY(h, Transfer::shared().copy(const_cast<double*>(data), h->d_pad, sizeof(double) * nc * h->V, false, h->device,
+  CUDA_TRY(h, transfers().copy(const_cast<double*>(data), h->d_pad, sizeof(double) * nc * h->V, false, h->device,
                                       h->stream));
   long long blocks = std::min<long long>((h->g.n + 255) / 256, 148 * 16);
   int prim = which == FGPU_PVAR;
@@ -2003,7 +2010,7 @@ int fgpu_download(fgpu_handle* h, int which, double* out, int64_t n) {
   B.npad = nc;
   if (int rc = launch_misc(h, 2, B)) return rc;
   if (int rc = launch_misc(h, 0, B)) return rc;
-  CUDA_TRY(h, Transfer::shared().copy(out, which == FGPU_PVAR ? B.out_p : B.out_c, sizeof(double) * nc * h->V, true,
+  CUDA_TRY(h, transfers().copy(out, which == FGPU_PVAR ? B.out_p : B.out_c, sizeof(double) * nc * h->V, true,
                                       h->device, h->stream));
   return FGPU_OK;
 }

@@ -41,10 +41,6 @@ class Transfer {
   static constexpr size_t kFreshDown = size_t(1) << 20, kDown = size_t(10) << 20, kUp = size_t(8) << 20;
   static constexpr int kLanes = 8, kDevices = 16;
 
-  static Transfer& shared() {
-    static Transfer* t = new Transfer;   // (never destroyed: no CUDA calls at process exit)
-    return *t;
-  }
   // Handles alive.  Neither waits for a transfer: one in flight belongs to a handle that is alive, so
   // that the lanes are not due.
   void attach() { ++handles_; }

@@ -292,3 +292,15 @@ def test_uploads_by_their_size(lib, n, lanes):
     assert t.copy(n, to_host=False) == 0
     assert (t.count(STREAMS) > 0) == lanes
     t.detach()
+
+
+@pytest.mark.parametrize("name", ["libfosite_gpu.so", "libfosite_gpu_exact.so"])
+def test_the_lanes_are_internal_to_a_library(name):
+    """Both builds in one process keep their own lanes: the object is not a unique symbol, which the dynamic
+    linker shares between all libraries that define it, of whatever version."""
+    path = os.path.join(os.path.dirname(CSRC), "lib", name)
+    if not os.path.exists(path) or not shutil.which("nm"):
+        pytest.skip("no library or no nm here")
+    names = subprocess.run(["nm", "-D", "--defined-only", path], check=True, capture_output=True, text=True).stdout
+    assert "fgpu_create" in names
+    assert not [n for n in names.splitlines() if " u " in n and "Transfer" in n]
