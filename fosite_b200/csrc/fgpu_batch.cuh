@@ -16,14 +16,12 @@ struct fgpu_batch {
   int nd = 2, order = 3;
   bool euler = false, prim = false;
   cudaStream_t stream = nullptr;
-  int variant = 0;               // stage layout: 0/6 the marching kernels (0: the base tile where they do
-                                 // not serve the batch), 2/3 shared-memory tiles
+  int variant = 0;               // stage layout: 0/6 the marching kernels, 2/3 shared-memory tiles
   StageArgs* d_args = nullptr;   // [order][n] step stages, then [n] RHS probes of the tuner
-  // marching layout: whether every stage of the batch can use it, the compiled-in limiter, the
+  // marching layout: the compiled-in limiter, the
   // block queue (2D: (member, first warp, has a tensor map, 0); 3D: (member, bx, by, bz)), rows per
   // warp (2D), and per argument table the tensor maps of the stage inputs, whether some member's
   // stage of a row reduces and whether every member's is a plain_stage
-  bool march = false;
   int march_lim = 0;
   int4* d_mqueue = nullptr;
   int nmqueue = 0;
@@ -89,7 +87,7 @@ int bset_err(fgpu_batch* b, int code, const std::string& msg) {
 bool in_table(const StageArgs* args, const StageArgs* t, size_t n) { return t && args >= t && args < t + n; }
 
 int launch_batched_stage(fgpu_batch* b, const StageArgs* args, int variant) {
-  if ((variant == 0 || variant == 6) && b->march) {
+  if (variant == 0 || variant == 6) {
     const size_t n = b->m.size();
     const bool e = in_table(args, b->d_eargs, (size_t)(b->stages + 2) * n);
     const fgpu_batch::MarchTable& T = e ? b->march_eargs : b->march_args;
@@ -104,8 +102,7 @@ int launch_batched_stage(fgpu_batch* b, const StageArgs* args, int variant) {
                        b->prim, b->march_lim, red, plain, args, maps, b->d_mqueue, b->nmqueue, b->stream));
     return FGPU_OK;
   }
-  if (variant == 6) variant = 0;
-  // the shared-memory base tile of the batch's tile queue: layouts 0, 2, 3
+  // the shared-memory tiles of the batch's tile queue
   if (b->nd == 2)
     BCUDA_TRY(b, legacy_batched_launch_2d(b->euler, b->prim, variant, args, b->d_tiles, b->ntiles, b->sms, b->stream));
   else
@@ -216,26 +213,26 @@ int upload_table(fgpu_batch* b, T** dst, const std::vector<T>& v) {
 
 // The marching layout's tables of rows of stage arguments (one entry per member and row): tensor
 // maps of the stage inputs, the kernel forms of each row; 2D arguments get the rows per warp.
-// Clears b->march when a member's stage cannot use the layout.
+// Every stage of an accepted member can use the layout (members have no accretion rows, and their
+// stage inputs are plain or formed states); one that could not is an error.
 int build_march_table(fgpu_batch* b, std::vector<StageArgs>& args, fgpu_batch::MarchTable& T) {
   const size_t n = b->m.size(), rows = args.size() / n;
   std::vector<CUtensorMap> maps(args.size());
   std::memset(maps.data(), 0, sizeof(CUtensorMap) * maps.size());
   T.red.assign(rows, 0);
   T.plain.assign(rows, 1);
-  for (size_t q = 0; q < args.size() && b->march; ++q) {
+  for (size_t q = 0; q < args.size(); ++q) {
     fgpu_handle* h = b->m[q % n];
     const StageArgs& A = args[q];
-    if (!tma_eligible(h, A)) b->march = false;
-    if (b->march && stage_has_tmap(h)) {
+    if (!tma_eligible(h, A)) return bset_err(b, FGPU_EUNSUPPORTED, "a member's stage that the batched kernels do not serve");
+    if (stage_has_tmap(h)) {
       const CUtensorMap* mp = stage_tmap(h, A.rin.base ? A.rin.base : A.in.base);
-      if (mp) maps[q] = *mp;
-      else b->march = false;
+      if (!mp) return bset_err(b, FGPU_ECUDA, "cuTensorMapEncodeTiled failed for a stage input");
+      maps[q] = *mp;
     }
     if (A.cfl_mode || A.last_stage || A.err_low) T.red[q / n] = 1;
     if (!plain_stage(A)) T.plain[q / n] = 0;
   }
-  if (!b->march) return FGPU_OK;
   if (b->nd == 2)
     for (auto& A : args) A.kchunk = b->march_rows;
   return upload_table(b, &T.d_maps, maps);
@@ -352,8 +349,7 @@ int build_embedded_tables(fgpu_batch* b) {
   b->ncblocks = (int)cblocks.size();
   if (int rc = upload_table(b, &b->d_ctlp, ctlp)) return rc;
   if (int rc = upload_table(b, &b->d_btp, btp)) return rc;
-  if (b->march)
-    if (int rc = build_march_table(b, eargs, b->march_eargs)) return rc;
+  if (int rc = build_march_table(b, eargs, b->march_eargs)) return rc;
   if (int rc = upload_table(b, &b->d_eargs, eargs)) return rc;
   if (int rc = upload_table(b, &b->d_fargs, fargs)) return rc;
   if (int rc = upload_table(b, &b->d_cargs, cargs)) return rc;
@@ -681,14 +677,11 @@ int fgpu_batch_create(fgpu_handle* const* members, int n, fgpu_batch** out) {
             for (int x = 0; x < tx; ++x) queue.push_back(make_int4(i | (stage_has_tmap(h) ? 1 << 30 : 0), x, y, z));
       }
     }
-    b->march = true;
     if (int rc = build_march_table(b, args, b->march_args)) return fail(rc, b->err);
-    if (b->march) {
-      if (int rc = upload_table(b, &b->d_mqueue, queue)) return fail(rc, b->err);
-      if (b->nd == 2) (b->euler ? strip2_batch_configure_euler : strip2_batch_configure_iso)(b->prim, b->march_lim);
-      else (b->euler ? march3_batch_configure_euler : march3_batch_configure_iso)(b->prim, b->march_lim);
-      b->nmqueue = (int)queue.size();
-    }
+    if (int rc = upload_table(b, &b->d_mqueue, queue)) return fail(rc, b->err);
+    if (b->nd == 2) (b->euler ? strip2_batch_configure_euler : strip2_batch_configure_iso)(b->prim, b->march_lim);
+    else (b->euler ? march3_batch_configure_euler : march3_batch_configure_iso)(b->prim, b->march_lim);
+    b->nmqueue = (int)queue.size();
   }
   cudaMemcpyAsync(b->d_args, args.data(), sizeof(StageArgs) * args.size(), cudaMemcpyHostToDevice, b->stream);
   cudaMemcpyAsync(b->d_bnd, bnd.data(), sizeof(BndArgs) * bnd.size(), cudaMemcpyHostToDevice, b->stream);
@@ -710,7 +703,6 @@ int fgpu_batch_create(fgpu_handle* const* members, int n, fgpu_batch** out) {
     b->nfwcb = (int)fwcb.size();
   }
   if (b->embedded) { if (int rc = build_embedded_tables(b)) return fail(rc, b->err); }
-  if (!b->march && b->variant == 6) b->variant = 0;
   *out = b;
   return FGPU_OK;
 }

@@ -20,8 +20,7 @@ cudaError_t legacy_stage_launch_2d(bool euler, bool prim, int variant, const Gri
                                    const StageArgs& A);
 cudaError_t legacy_stage_launch_3d(bool euler, bool prim, int variant, const Grid& g, int kchunk, cudaStream_t s,
                                    const StageArgs& A);
-// Batches: layouts 0, 2, 3 (any other id: 0) over the tile queue (grid, bx, by, bz) of base
-// tiles, one persistent launch sized by the occupancy calculator for `sms` SMs.
+// Batches: layouts 2 and 3 over the tile queue (grid, bx, by, bz) of base tiles, one persistent launch sized by the occupancy calculator for `sms` SMs.
 cudaError_t legacy_batched_launch_2d(bool euler, bool prim, int variant, const StageArgs* args, const int4* tiles,
                                      int ntiles, int sms, cudaStream_t s);
 cudaError_t legacy_batched_launch_3d(bool euler, bool prim, int variant, const StageArgs* args, const int4* tiles,

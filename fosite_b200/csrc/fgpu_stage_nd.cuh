@@ -15,10 +15,11 @@ template <int ND, bool EU, bool PRIM, int TX, int TY, int MINB>
 struct TileLayout {
   static constexpr size_t SMEM = stage_smem_bytes<Phys<ND, EU>::V, TX, TY>();
   // the tiles use more than the default 48 KB of dynamic shared memory: opt in (per device)
-  static void configure(bool batched) {
+  template <bool BATCHED>
+  static void configure() {
     cudaFuncSetAttribute(stage_kernel<ND, EU, PRIM, TX, TY, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)SMEM);
-    if (batched)
+    if constexpr (BATCHED)
       cudaFuncSetAttribute(batched_stage_kernel<ND, EU, PRIM, TX, TY, MINB>,
                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
   }
@@ -44,11 +45,11 @@ template <> struct TileShapes<3> { static constexpr int TY = kBaseTY3, M2 = 4, M
 template <int ND, bool EU, bool PRIM>
 void configure_t() {
   using S = TileShapes<ND>;
-  TileLayout<ND, EU, PRIM, 32, S::TY, 1>::configure(true);
-  TileLayout<ND, EU, PRIM, 32, S::TY, S::M2>::configure(true);
-  TileLayout<ND, EU, PRIM, 32, S::TY, S::M3>::configure(true);
-  TileLayout<ND, EU, PRIM, 32, S::TY4, S::M4>::configure(false);
-  TileLayout<ND, EU, PRIM, 32, S::TY4, S::M5>::configure(false);
+  TileLayout<ND, EU, PRIM, 32, S::TY, 1>::template configure<false>();
+  TileLayout<ND, EU, PRIM, 32, S::TY, S::M2>::template configure<true>();
+  TileLayout<ND, EU, PRIM, 32, S::TY, S::M3>::template configure<true>();
+  TileLayout<ND, EU, PRIM, 32, S::TY4, S::M4>::template configure<false>();
+  TileLayout<ND, EU, PRIM, 32, S::TY4, S::M5>::template configure<false>();
 }
 
 template <int ND, bool EU, bool PRIM>
@@ -75,8 +76,7 @@ template <int ND, bool EU, bool PRIM>
 void batched_t(int variant, const StageArgs* args, const int4* tiles, int ntiles, int sms, cudaStream_t s) {
   using S = TileShapes<ND>;
   if (variant == 2) TileLayout<ND, EU, PRIM, 32, S::TY, S::M2>::launch_batched(args, tiles, ntiles, sms, s);
-  else if (variant == 3) TileLayout<ND, EU, PRIM, 32, S::TY, S::M3>::launch_batched(args, tiles, ntiles, sms, s);
-  else TileLayout<ND, EU, PRIM, 32, S::TY, 1>::launch_batched(args, tiles, ntiles, sms, s);
+  else TileLayout<ND, EU, PRIM, 32, S::TY, S::M3>::launch_batched(args, tiles, ntiles, sms, s);
 }
 
 template <int ND>
