@@ -55,9 +55,9 @@ def test_disk_ensemble_matches_single_grids(exact):
 
 @pytest.mark.parametrize("exact,tpb", [(True, None), (False, None), (True, 3)])
 def test_disk_ensemble_tma_layout(exact, tpb, monkeypatch):
-    """The TMA-staged batched layout (6, one block per column of tiles, tensor maps of every
-    member's stage inputs in a device table): every member equals its lone run on the TMA
-    layout bit for bit, and on the exact build also its lone run on the base tile."""
+    """The marching batched layout (6, four warps of rows a block, tensor maps of every member's stage
+    inputs in a device table): every member equals its lone run on that layout bit for bit, and on
+    the exact build also its lone run on a shared-memory tile (2)."""
     from fosite_b200.sim import Batch
     monkeypatch.setenv("FGPU_STAGE_VARIANT", "6")
     if tpb:
@@ -65,7 +65,7 @@ def test_disk_ensemble_tma_layout(exact, tpb, monkeypatch):
     specs = _disk_specs(7)
     members = [_disk_member(*sp, exact=exact) for sp in specs]
     alone = [_disk_member(*sp, exact=exact) for sp in specs]
-    monkeypatch.setenv("FGPU_STAGE_VARIANT", "0")
+    monkeypatch.setenv("FGPU_STAGE_VARIANT", "2")
     base = [_disk_member(*sp, exact=exact) for sp in specs] if exact else []
     b = Batch(members)
     assert b.layout() == 6
@@ -84,7 +84,7 @@ def test_disk_ensemble_tma_layout(exact, tpb, monkeypatch):
 @pytest.mark.parametrize("limiters", [(abi.VANLEER, abi.VANLEER, abi.VANLEER),
                                       (abi.MINMOD, abi.MONOCENT, abi.VANLEER)])
 def test_euler2d_tma_batch_limiters_and_autotune(limiters, monkeypatch):
-    """Euler members on the TMA batched layout with one compiled-in limiter, and with mixed
+    """Euler members on the marching batched layout with one compiled-in limiter, and with mixed
     limiters (MC with theta 1.3 among them: the kernel reads limiter and theta per member);
     the tuner's pick keeps every result."""
     from fosite_b200.sim import Batch, Simulation

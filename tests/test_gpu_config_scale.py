@@ -65,7 +65,7 @@ def _check_status(g, pin, tag):
 @pytest.mark.parametrize("variant,tpb", [(None, None), (4, None), (6, None), (6, 4)])
 def test_khi256_bitwise_1000_steps(variant, tpb, monkeypatch):
     """KHI 256^2, SSPRK3: the exact build's state after 1 and 1000 steps is the oracle's bit for
-    bit (tuned layout, shared-memory tile, TMA-staged tile, TMA tiles in columns of four)."""
+    bit (tuned layout, shared-memory tile, marching strips by the grid's rule and of 32 rows a warp)."""
     pin = _pin("khi256")
     if tpb:
         monkeypatch.setenv("FGPU_TMA_TPB", str(tpb))
@@ -109,7 +109,7 @@ def test_khi256_product_build_and_conservation():
 @pytest.mark.parametrize("exact,variant", [(True, None), (False, None), (True, 6), (False, 7)])
 def test_disk512_fargo(exact, variant, monkeypatch):
     """Logcylindrical isothermal disk 512x1024 with FARGO and absorbing radial boundaries (tuned
-    layout, and the TMA-staged tiles with their frame changes): one step against the oracle run
+    layout, and the marching strips with their frame changes): one step against the oracle run
     here, 2000 steps against the pinned rows."""
     pin = _pin("disk512")
     cfg, p, extra = problems.disk2d(nr=512, nphi=1024, fargo=1)

@@ -1,13 +1,13 @@
 """Stage-kernel tile layouts against the CPU oracle.
 
-The stage kernel comes in several tile layouts (shared-memory tiles 0/2/3/4/5, the
-warp-shuffle window 1, the tile whose halo planes arrive by TMA bulk tensor copies 6),
-picked per grid by the tuner; FGPU_STAGE_VARIANT / FGPU_KCHUNK force one.  Every layout
-must give the oracle's numbers bit for bit on the --fmad=false build, and the product
-build must stay within 1e-12 relative L1 of it.  The TMA layout applies FARGO's frame
-changes where it converts the staged points; launches it does not serve (viscosity,
-accretion, odd x extent) run on layout 0, and those cases check that the fallback keeps
-the results too.
+The stage kernel comes in several layouts (shared-memory tiles 2/3/4/5, the warp-shuffle
+window 1, and the marching kernels 6: 2D strips of columns, 3D tiles marching in z, which are also
+what 0, the default, launches), picked per grid by the tuner; FGPU_STAGE_VARIANT / FGPU_KCHUNK
+force one.  Every layout must give the oracle's numbers bit for bit on the --fmad=false build, and
+the product build must stay within 1e-12 relative L1 of it.  The marching kernels apply FARGO's
+frame changes where they convert the staged points; launches that they do not serve (accretion,
+interface fluxes, stage states summed at the stencil points) run on the base tile, and those cases
+check that the fallback keeps the results too.
 """
 import numpy as np
 import pytest
@@ -27,11 +27,8 @@ def _force(monkeypatch, variant, kchunk=None):
         monkeypatch.delenv("FGPU_KCHUNK", raising=False)
 
 
-@pytest.mark.gpu
-@pytest.mark.parametrize("name", sorted(CASES))
-def test_tma_layout_bitwise(name, monkeypatch):
-    """RHS, FirstStep's dt and four steps of the TMA layout equal the oracle's bit for bit."""
-    _force(monkeypatch, 6, 4)
+def _bitwise(name):
+    """RHS, FirstStep's dt and four steps equal the oracle's bit for bit."""
     cfg, o, g = _pair(name, exact=True)
     tol = 1e-13 if _inexact(cfg) else 0.0
     o.compute_rhs()
@@ -62,10 +59,26 @@ def test_tma_layout_bitwise(name, monkeypatch):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("name", sorted(CASES))
+def test_tma_layout_bitwise(name, monkeypatch):
+    """The marching kernels, whose planes and rows arrive by TMA, on every case."""
+    _force(monkeypatch, 6, 4)
+    _bitwise(name)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", sorted(CASES))
+def test_shared_memory_tile_bitwise(name, monkeypatch):
+    """The shared-memory tile on every case (the tile that layout 0 was before the marching kernels, with
+    a register cap)."""
+    _force(monkeypatch, 2, 4)
+    _bitwise(name)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", sorted(CASES))
 def test_tma_2d_tile_columns_bitwise(name, monkeypatch):
-    """2D blocks computing columns of three TMA tiles (the next tile's box in flight, the last
-    column partial where the tile rows do not divide): four steps equal the oracle's bit for
-    bit on the exact build."""
+    """2D strips of 24 rows a warp (the last one partial where the rows do not divide): four steps equal
+    the oracle's bit for bit on the exact build."""
     _force(monkeypatch, 6)
     monkeypatch.setenv("FGPU_TMA_TPB", "3")
     cfg, o, g = _pair(name, exact=True)
@@ -150,13 +163,13 @@ def test_multi_tile_3d_product_build(variant, monkeypatch):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("name", ["khi_ssprk3_mc_prim", "disk_logcyl_pointmass", "iso_axis_cyl3d"])
-@pytest.mark.parametrize("variant", [0, 6])
+@pytest.mark.parametrize("variant", [0, 2, 6])
 @pytest.mark.parametrize("exact", [True, False])
 def test_shu_osher_formed_primitive_states(name, variant, exact, monkeypatch):
     """Fixed-step Shu-Osher with primitive reconstruction: stages 1 and 2 also write the
     primitive variables of their results, which the next stage reads ready-made; the states
     after six steps equal those of converting every staged point (FGPU_FORM_SO=0) bit for bit,
-    on the shared-memory and the TMA-staged tiles, exact and product builds."""
+    on the marching kernels (0, 6) and the shared-memory tile (2), exact and product builds."""
     from fosite_b200.sim import Simulation
     _force(monkeypatch, variant)
     out = []
