@@ -438,7 +438,7 @@ __device__ __forceinline__ void stage_cell_epilogue(const StageArgs& A, const in
       if (EU && A.cfl_roundtrip) p[V - 1] = dmax(p[V - 1], P.pmin);
       double cs = EU ? PH::cs_of(p, P) : __ldg(M.cs + ip);
       double v3[4];
-      CE::cfl_cell(p, cs, M, ip, v3);
+      CE::template cfl_cell<true>(p, cs, M, ip, v3);
 #pragma unroll
       for (int q = 0; q < 4; ++q) cflv[q] = dmax(cflv[q], v3[q]);
       if (EU && A.cfl_roundtrip) PH::p2c(p, c, P);
@@ -467,7 +467,7 @@ __device__ __forceinline__ void stage_cell_epilogue(const StageArgs& A, const in
     double cs = EU ? PH::cs_of(pc, P) : __ldg(M.cs + ip);
     if (A.cfl_mode == 2) {
       double v3[4];
-      CE::cfl_cell(pc, cs, M, ip, v3);
+      CE::template cfl_cell<true>(pc, cs, M, ip, v3);
 #pragma unroll
       for (int q = 0; q < 4; ++q) cflv[q] = dmax(cflv[q], v3[q]);
     }

@@ -374,7 +374,7 @@ __global__ void __launch_bounds__(32 * NW, 2) stage2_kernel(const __grid_constan
           if (EU && A.cfl_roundtrip) p[V - 1] = dmax(p[V - 1], P.pmin);
           double cs = EU ? PH::cs_of(p, P) : M.cs[ip];
           double v3[4];
-          CE::cfl_cell(p, cs, M, ip, v3);
+          CE::template cfl_cell<true>(p, cs, M, ip, v3);
 #pragma unroll
           for (int q = 0; q < 3; ++q) cflv[q] = dmax(cflv[q], v3[q]);
           if (EU && A.cfl_roundtrip) PH::p2c(p, cv, P);
@@ -396,7 +396,7 @@ __global__ void __launch_bounds__(32 * NW, 2) stage2_kernel(const __grid_constan
       if (A.cfl_mode == 2) {
         double cs = EU ? PH::cs_of(pc, P) : M.cs[ip];
         double v3[4];
-        CE::cfl_cell(pc, cs, M, ip, v3);
+        CE::template cfl_cell<true>(pc, cs, M, ip, v3);
 #pragma unroll
         for (int q = 0; q < 3; ++q) cflv[q] = dmax(cflv[q], v3[q]);
         if ((A.checkdata & 0x01) && !(cs > 0.)) flags |= 0x01;
