@@ -224,7 +224,7 @@ int build_march_table(fgpu_batch* b, std::vector<StageArgs>& args, fgpu_batch::M
   for (size_t q = 0; q < args.size(); ++q) {
     fgpu_handle* h = b->m[q % n];
     const StageArgs& A = args[q];
-    if (!tma_eligible(h, A)) return bset_err(b, FGPU_EUNSUPPORTED, "a member's stage that the batched kernels do not serve");
+    if (!march_eligible(h, A)) return bset_err(b, FGPU_EUNSUPPORTED, "a member's stage that the batched kernels do not serve");
     if (stage_has_tmap(h)) {
       const CUtensorMap* mp = stage_tmap(h, A.rin.base ? A.rin.base : A.in.base);
       if (!mp) return bset_err(b, FGPU_ECUDA, "cuTensorMapEncodeTiled failed for a stage input");
@@ -670,7 +670,7 @@ int fgpu_batch_create(fgpu_handle* const* members, int n, fgpu_batch** out) {
         const int warps = strips(g) * ((g.ny + b->march_rows - 1) / b->march_rows);
         for (int w = 0; w < warps; w += kStripWarps) queue.push_back(make_int4(i, w, stage_has_tmap(h) ? 1 : 0, 0));
       } else {
-        const int tx = (g.nx + kTmaTX - 1) / kTmaTX, ty = (g.ny + kTmaTY - 1) / kTmaTY;
+        const int tx = (g.nx + kMarchTX - 1) / kMarchTX, ty = (g.ny + kMarchTY - 1) / kMarchTY;
         const int tz = (g.nz + h->kchunk - 1) / h->kchunk;
         for (int z = 0; z < tz; ++z)
           for (int y = 0; y < ty; ++y)

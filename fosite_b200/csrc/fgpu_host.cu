@@ -176,8 +176,8 @@ struct fgpu_handle {
   bool so_form = false;
   double* d_pform[2] = {nullptr, nullptr};
   double* d_ready = nullptr;    // ... into this array (one state)
-  int variant = 0;              // stage kernel layout: 0 the default, the marching kernels wherever they
-                                // serve the stage, else the shared-memory base tile; 1 warp-shuffle window,
+  int variant = 0;              // stage kernel layout: 0 the marching kernels wherever they serve the
+                                // stage, else the shared-memory base tile; 1 warp-shuffle window,
                                 // 2/3 tile with a register cap for more resident blocks, 4 taller tile,
                                 // 6 marching kernels (2D fgpu_strip2.cuh, 3D fgpu_march3.cuh), 7 the 2D
                                 // strips with half the rows per warp
@@ -485,7 +485,7 @@ const CUtensorMap* stage_tmap(fgpu_handle* h, const double* base) {
     rank = 4;
     dims[0] = g.nx; dims[1] = g.ny; dims[2] = g.nz; dims[3] = h->V;
     strides[0] = 8ull * g.nx; strides[1] = 8ull * g.nx * g.ny; strides[2] = 8ull * g.n;
-    box[0] = kTmaTX + 4; box[1] = kTmaTY + 4; box[2] = 1; box[3] = h->V;
+    box[0] = kMarchTX + 4; box[1] = kMarchTY + 4; box[2] = 1; box[3] = h->V;
   } else {
     rank = 3;
     dims[0] = g.nx; dims[1] = g.ny; dims[2] = h->V;
@@ -503,7 +503,7 @@ const CUtensorMap* stage_tmap(fgpu_handle* h, const double* base) {
 // The marching layouts serve stages whose input is a plain or formed state (no k-sums at the
 // stencil points) without accretion rows or interface-flux output; FARGO frame changes on 2D
 // meshes, where they apply to the staged points of a plain input.
-bool tma_eligible(const fgpu_handle* h, const StageArgs& A) {
+bool march_eligible(const fgpu_handle* h, const StageArgs& A) {
   const StateRef& S = A.rin.base ? A.rin : A.in;
   const bool frames = h->fargo || A.w_sub || S.pre.n || A.in.pre.n || A.yn_chain.n || A.y0_chain.n || A.err_chain.n;
   return (!frames || h->nd == 2) && !A.brow && !A.flux_out && S.nk == 0 && (S.pre.n == 0 || &S == &A.in);
@@ -516,7 +516,7 @@ template <int ND, bool EU, bool PRIM>
 int launch_stage_t(fgpu_handle* h, StageArgs& A) {
   A.kchunk = h->kchunk;
   const Grid& g = h->g;
-  if ((h->variant == 0 || h->variant >= 6) && tma_eligible(h, A)) {
+  if ((h->variant == 0 || h->variant >= 6) && march_eligible(h, A)) {
     const StateRef& SR = A.rin.base ? A.rin : A.in;
     const int lim = compiled_limiter(A.limiter, A.constant_recon != 0, A.theta);
     const bool tma = stage_has_tmap(h);
@@ -1708,10 +1708,11 @@ int fgpu_create(const fgpu_config* cfg, int device, fgpu_handle** out) {
     // FGPU_STAGE_VARIANT / FGPU_KCHUNK force a stage-kernel layout and z chunk (the tuner's choice otherwise)
     // Default layout: the marching kernels (0).  2D isothermal grids start with the register-capped
     // shared-memory tile (3): their rows carry a third less arithmetic while the opening of a warp's
-    // chunk costs the same, so that small disks are faster on tiles (186 x 390: 44 against 52 us a
-    // step), 512 x 1024 with FARGO is a draw (195 us), and only large ones gain from marching (48
-    // disks in one batch, 5 million cells: 950 against 1430 us), which the tuner finds.  One layout for
-    // all of them, so that a batch and its members' lone runs keep the same bits.
+    // chunk costs the same, so that small disks are faster on tiles (186 x 390: 46 against 53 us a
+    // step; with FARGO 79 against 91).  Larger ones gain from marching (256 x 512 66 against 57 us, 512 x
+    // 1024 139 / 119, with FARGO 196 / 198, 2048^2 960 / 670; 48 disks in one batch, 5 million cells, 1280 /
+    // 920), which the tuner finds: a batch starts with its members' layout, and one layout for all of
+    // them keeps a batch and its members' lone runs at the same bits.
     h->variant = (!h->euler && h->nd == 2) ? 3 : 0;
     if (const char* e = std::getenv("FGPU_STAGE_VARIANT")) h->variant = std::max(0, std::min(7, std::atoi(e)));
     if (const char* e = std::getenv("FGPU_KCHUNK")) { int v = std::atoi(e); if (v > 0) h->kchunk = v; }

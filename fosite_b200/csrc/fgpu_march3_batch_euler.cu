@@ -10,11 +10,11 @@ template <bool PRIM>
 struct March {
   template <int LIM, bool RED, bool SRC>
   struct K {
-    static constexpr auto kernel = batched_march3_kernel<true, PRIM, kTmaTX, kTmaTY, 2, LIM, RED, SRC>;
-    static constexpr size_t SMEM = March3Layout<Phys<3, true>::V, kTmaTX, kTmaTY>::SMEM;
+    static constexpr auto kernel = batched_march3_kernel<true, PRIM, kMarchTX, kMarchTY, 2, LIM, RED, SRC>;
+    static constexpr size_t SMEM = March3Layout<Phys<3, true>::V, kMarchTX, kMarchTY>::SMEM;
     static void configure() { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM); }
     static void run(const StageArgs* args, const CUtensorMap* maps, const int4* queue, int nblocks, cudaStream_t s) {
-      kernel<<<nblocks, kTmaTX * kTmaTY, SMEM, s>>>(args, maps, queue);
+      kernel<<<nblocks, kMarchTX * kMarchTY, SMEM, s>>>(args, maps, queue);
     }
   };
 };

@@ -11,13 +11,13 @@ template <bool PRIM>
 struct March {
   template <int LIM, bool RED, bool SRC>
   struct K {
-    static constexpr auto kernel = march3_kernel<true, PRIM, kTmaTX, kTmaTY, kMinBlocks, LIM, RED, SRC>;
-    static constexpr size_t SMEM = March3Layout<Phys<3, true>::V, kTmaTX, kTmaTY>::SMEM;
+    static constexpr auto kernel = march3_kernel<true, PRIM, kMarchTX, kMarchTY, kMinBlocks, LIM, RED, SRC>;
+    static constexpr size_t SMEM = March3Layout<Phys<3, true>::V, kMarchTX, kMarchTY>::SMEM;
     static void configure() { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM); }
     static void run(int kchunk, cudaStream_t s, const StageArgs* A, const CUtensorMap* map, bool tma) {
       const Grid& g = A->g;
-      const dim3 grid((g.nx + kTmaTX - 1) / kTmaTX, (g.ny + kTmaTY - 1) / kTmaTY, (g.nz + kchunk - 1) / kchunk);
-      kernel<<<grid, kTmaTX * kTmaTY, SMEM, s>>>(*A, *map, tma ? 1 : 0);
+      const dim3 grid((g.nx + kMarchTX - 1) / kMarchTX, (g.ny + kMarchTY - 1) / kMarchTY, (g.nz + kchunk - 1) / kchunk);
+      kernel<<<grid, kMarchTX * kMarchTY, SMEM, s>>>(*A, *map, tma ? 1 : 0);
     }
   };
 };

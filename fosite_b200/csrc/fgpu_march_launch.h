@@ -13,7 +13,7 @@
 namespace fgpu {
 
 // 3D tile: 32 x 8 cells, two 256-thread blocks per SM
-constexpr int kTmaTX = 32, kTmaTY = 8;
+constexpr int kMarchTX = 32, kMarchTY = 8;
 // 2D: warps per block and resident blocks per SM (16 warps of 128 registers)
 constexpr int kStripWarps = 4, kStripMinBlocks = 4;
 constexpr int kStripW = 30;   // columns of a warp's strip
@@ -74,7 +74,7 @@ inline long long strip_warp_rows(const Grid& g) { return (long long)((g.nx + kSt
 // planes takes about c + 2 plane times (its opening), so the chunk that minimises waves x (c + 2).
 // 90 x 75 x 61: chunks of 4 / 8 / 16 planes 571 / 535 / 835 us a Dormand-Prince step.
 inline int march_chunk(const Grid& g, int copies) {
-  const long long tiles = (long long)copies * ((g.nx + kTmaTX - 1) / kTmaTX) * ((g.ny + kTmaTY - 1) / kTmaTY);
+  const long long tiles = (long long)copies * ((g.nx + kMarchTX - 1) / kMarchTX) * ((g.ny + kMarchTY - 1) / kMarchTY);
   int best = 1;
   double least = 1e300;
   for (int c = 1; c <= 64 && c <= g.nz; ++c) {

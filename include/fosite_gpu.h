@@ -282,9 +282,9 @@ int fgpu_set_output_time(fgpu_handle* h, double tout);
  * counterpart in the reference. */
 int fgpu_autotune(fgpu_handle* h, int reps, int* variant);
 /* The stage-kernel layout later steps use (the tuner's choice, FGPU_STAGE_VARIANT, or
- * the default 0: the marching kernels wherever they serve the stage, else the shared-memory
- * base tile) and, for 3D grids, the z extent one block marches through.  Either
- * pointer may be NULL.  No counterpart in the reference. */
+ * the default: 0, the marching kernels wherever they serve the stage, else the shared-memory
+ * base tile; 3, a shared-memory tile, for 2D isothermal grids) and, for 3D grids, the z extent
+ * one block marches through.  Either pointer may be NULL.  No counterpart in the reference. */
 int fgpu_stage_layout(const fgpu_handle* h, int* variant, int* kchunk);
 
 /* ---- batched ensembles (no counterpart in the reference, which integrates one
