@@ -266,8 +266,8 @@ struct Phys {
   // GetSoundSpeed (physics_euler.f90:2682-2689): sqrt(MAX(2 TINY, gamma*p/rho)).
   // The product build evaluates sqrt(s/rho) as s*rsqrt(s*rho) with s = gamma*p (within a few
   // ulp).  Wherever s*rho leaves the normal range, or s or rho is not positive, that form gives
-  // a NaN, an infinity, a negative value or one below the floor sqrt(2 TINY) = 2^-510.5 (cs_good); the
-  // reference's form then takes over.
+  // a NaN, an infinity, a negative value or one below the floor sqrt(2 TINY) = 2^-510.5; the
+  // reference's form then takes over (cs_good), as it does where s/rho leaves the range upwards.
   static __device__ __forceinline__ double cs_of(const double* p, const PhysP& P) {
 #ifdef FGPU_EXACT
     return sqrt(dmax(P.tiny2, P.gamma * p[V - 1] / p[0]));
@@ -282,8 +282,8 @@ struct Phys {
     const double s = P.gamma * p[V - 1];
     return s * rsqrt_refined(s * p[0]);
   }
-  // at least 2^-510, finite
-  static __device__ __forceinline__ bool cs_good(double cs) { return in_range<510, 1024>(cs); }
+  // at least 2^-510 and below 2^512, where s/rho overflows and the reference's sound speed is infinite
+  static __device__ __forceinline__ bool cs_good(double cs) { return in_range<510, 512>(cs); }
 #endif
 };
 

@@ -9,7 +9,7 @@ import numpy as np
 import pytest
 
 from fosite_b200 import abi, build
-from cases import _visc
+from cases import _gauss3d, _khi, _visc
 
 SRC = r'''
 #include "fgpu_device.cuh"
@@ -133,3 +133,23 @@ def test_stresses_of_a_ghost_cell_without_width():
         assert np.array_equal(kind(a), kind(b))
     m = np.isfinite(a)
     assert np.abs(a[m] - b[m]).sum() <= 1e-12 * np.abs(a[m]).sum()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("case", [_khi(n=(33, 20)), _khi(n=(40, 22), variables=abi.PRIMITIVE, limiter=abi.MINMOD),
+                                  _gauss3d(n=(34, 12, 9), method=abi.MODIFIED_EULER, tdorder=3)], ids=["cons", "prim", "3d"])
+def test_sound_speeds_that_overflow(case):
+    """A subnormal density: p/rho is infinite, and so is the sound speed; the time step is 0 and the start
+    refused as by the oracle (s rsqrt(s rho) is 2e154 there)."""
+    from fosite_b200.sim import Simulation
+    pyoracle = pytest.importorskip("pyoracle")
+    cfg, p, _ = case
+    p = p.copy()
+    p[0, p.shape[1] // 2, 9:11, 12:15] = 1e-308
+    p[-1, p.shape[1] // 2, 9:11, 12:15] = 2.5
+    o, g = pyoracle.Oracle(cfg), Simulation(cfg)
+    for s in (o, g):
+        s.set_state(abi.PVAR, p)
+    assert g.calc_timestep() == 0.0
+    assert g.first_step() == o.first_step() and g.status().dt == o.status().dt == 0.0
+    g.close()
