@@ -9,10 +9,10 @@
 // cost (2 MiB in all 2 ms, 32 MiB 18 ms; freeing them 4 ms), so a slot holds the pieces asked
 // of it so far (256 KiB for transfers up to 4 MiB, 4 MiB from 32 MiB on), and the lanes outlive the
 // handles: a program that opens, reads and closes one grid after another keeps them (freed with every
-// last handle they cost 35 ms a 256^2 grid).  The slots serve every device, each of which has its own
-// streams, so that handles on two devices transfer in turn as those of one.  The lanes are given back
-// when the last handle goes and no transfer has used them since the previous time that it went; at
-// most 32 MiB and eight streams a device stay.
+// last handle they cost 35 ms a 256^2 grid).  Each device has lanes of its own, so that handles on two
+// devices transfer in turn as those of one; they belong to its context, and go unused once a program has
+// reset that between two grids.  The lanes are given back when the last handle goes and no transfer
+// has used them since the previous time that it went; at most 32 MiB and eight streams a device stay.
 // Pinned host memory, transfers below the thresholds, and calls that find the lanes in use or cannot
 // make them (devices past the kDevices-th too) take the driver's path.  Thresholds, by what bounds
 // the driver's one core (16 host cores, ms, driver / lanes):
@@ -68,14 +68,14 @@ class Transfer {
     used_ = true;
     cudaError_t e = cudaEventRecord(D->ready, s);   // the lanes start after the work enqueued on s
     if (e != cudaSuccess) return e;
-    const size_t piece = std::min(slot_bytes_, piece_bytes(bytes, D->lanes));
+    const size_t piece = std::min(D->slot_bytes, piece_bytes(bytes, D->lanes));
     const size_t pieces = (bytes + piece - 1) / piece;
     const int n = (int)std::min<size_t>(D->lanes, pieces);
     cudaError_t err[kLanes] = {};
     const cudaStreamCaptureMode capture = capture_mode();
     auto work = [&](int t) {
       const cudaStream_t stream = D->stream[t];
-      char* const slot = slots_ + t * slot_bytes_;
+      char* const slot = D->slots + t * D->slot_bytes;
       cudaStreamCaptureMode mode = capture;   // the lane's threads wait under the caller's rules
       cudaError_t r = cudaThreadExchangeStreamCaptureMode(&mode);
       if (r == cudaSuccess) r = cudaSetDevice(device);
@@ -107,6 +107,9 @@ class Transfer {
  private:
   struct Device {
     int id = -1, lanes = 0;
+    unsigned long long context = 0;   // what the rest belongs to
+    char* slots = nullptr;            // one pinned block, a slot of slot_bytes per lane
+    size_t slot_bytes = 0;
     cudaStream_t stream[kLanes] = {};
     cudaEvent_t ready = nullptr;
   };
@@ -117,7 +120,7 @@ class Transfer {
   struct OnDevice {   // the calling thread's device for the length of a transfer
     int before = -1;
     explicit OnDevice(int device) {
-      if (device >= 0 && cudaGetDevice(&before) == cudaSuccess && before != device) cudaSetDevice(device);
+      if (device >= 0 && cudaGetDevice(&before) == cudaSuccess) cudaSetDevice(device);   // (makes its context current)
     }
     ~OnDevice() {
       if (before >= 0) cudaSetDevice(before);
@@ -125,8 +128,6 @@ class Transfer {
   };
   std::mutex mutex_;
   Device devices_[kDevices];   // those with lanes first
-  char* slots_ = nullptr;      // one pinned block, kLanes slots of slot_bytes_
-  size_t slot_bytes_ = 0;
   std::atomic<long long> handles_{0};
   bool used_ = false;          // since the last handle last went
 
@@ -159,46 +160,76 @@ class Transfer {
     cudaThreadExchangeStreamCaptureMode(&mode);
     return callers;
   }
-  static int lane_count() { return std::max(1, std::min<int>(kLanes, (int)std::thread::hardware_concurrency() / 2)); }
-  // the lanes of the current device with slots for pieces of a transfer of `bytes`, or smaller
-  // slots where no larger ones are to be had
+  // Driver calls: the identity of the current context (never used twice in a process), and whether a
+  // device's context exists (cudaSetDevice would make one).
+  static unsigned long long current_context() {
+    static int (*const get_id)(void*, unsigned long long*) =
+        reinterpret_cast<int (*)(void*, unsigned long long*)>(driver_call("cuCtxGetId"));
+    unsigned long long id = 0;
+    return get_id && get_id(nullptr, &id) == 0 ? id : 0;
+  }
+  static bool has_context(int device) {
+    static int (*const get_state)(int, unsigned*, int*) =
+        reinterpret_cast<int (*)(int, unsigned*, int*)>(driver_call("cuDevicePrimaryCtxGetState"));
+    unsigned flags = 0;
+    int active = 1;
+    return !get_state || get_state(device, &flags, &active) != 0 || active != 0;
+  }
+  static void* driver_call(const char* name) {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPoint(name, &p, cudaEnableDefault, &found) != cudaSuccess) cudaGetLastError();
+    return p;
+  }
+  // the lanes of the current device and context with slots for pieces of a transfer of `bytes`, or
+  // smaller slots where no larger ones are to be had
   Device* prepare(int device, size_t bytes) {
+    const unsigned long long context = current_context();
     Device* D = devices_;
-    while (D < devices_ + kDevices && D->id >= 0 && D->id != device) ++D;
+    while (D < devices_ + kDevices && D->id >= 0 && (D->id != device || D->context != context)) ++D;
     if (D == devices_ + kDevices) return nullptr;
     if (D->id < 0) {
+      const int want = std::max(1, std::min<int>(kLanes, (int)std::thread::hardware_concurrency() / 2));
       if (cudaEventCreateWithFlags(&D->ready, cudaEventDisableTiming) != cudaSuccess) D->ready = nullptr;
-      while (D->ready && D->lanes < lane_count() &&
+      while (D->ready && D->lanes < want &&
              cudaStreamCreateWithFlags(&D->stream[D->lanes], cudaStreamNonBlocking) == cudaSuccess)
         ++D->lanes;
-      if (D->lanes) D->id = device;
-      else release(*D);
+      if (D->lanes) {
+        D->id = device;
+        D->context = context;
+      } else {
+        free_lanes(*D);
+        *D = Device();
+      }
     }
-    if (D->lanes) reserve(piece_bytes(bytes, D->lanes));
+    if (D->lanes) reserve(*D, piece_bytes(bytes, D->lanes));
     cudaGetLastError();
-    return D->lanes && slots_ ? D : nullptr;
+    return D->slots ? D : nullptr;
   }
-  void reserve(size_t piece) {
+  static void reserve(Device& D, size_t piece) {
     size_t want = kLeast;
     while (want < piece) want *= 2;
     char* block = nullptr;
-    if (want <= slot_bytes_ ||
-        cudaHostAlloc(reinterpret_cast<void**>(&block), want * lane_count(), cudaHostAllocPortable) != cudaSuccess)
-      return;
-    if (slots_) cudaFreeHost(slots_);
-    slots_ = block;
-    slot_bytes_ = want;
+    if (want <= D.slot_bytes || cudaMallocHost(reinterpret_cast<void**>(&block), want * D.lanes) != cudaSuccess) return;
+    if (D.slots) cudaFreeHost(D.slots);
+    D.slots = block;
+    D.slot_bytes = want;
   }
-  static void release(Device& D) {
+  static void free_lanes(Device& D) {
     for (int t = 0; t < D.lanes; ++t) cudaStreamDestroy(D.stream[t]);
     if (D.ready) cudaEventDestroy(D.ready);
-    D = Device();
+    if (D.slots) cudaFreeHost(D.slots);
   }
+  // gives the lanes back; those of a context that is gone went with it
   void release() {
-    for (Device& D : devices_) release(D);
-    if (slots_) cudaFreeHost(slots_);
-    slots_ = nullptr;
-    slot_bytes_ = 0;
+    for (Device& D : devices_) {
+      if (D.id >= 0 && has_context(D.id)) {
+        const OnDevice on(D.id);
+        if (current_context() == D.context) free_lanes(D);
+        cudaGetLastError();
+      }
+      D = Device();
+    }
   }
 };
 

@@ -110,3 +110,48 @@ def test_transfer_while_another_thread_captures(n):
     assert got == [0, 0]
     assert np.array_equal(_interior(back, s.cfg), _interior(c, s.cfg))
     s.close()
+
+
+_RESET = """
+import sys
+import ctypes as C
+import numpy as np
+from fosite_b200 import abi, problems
+from fosite_b200.sim import Simulation
+
+runtime = C.CDLL(sys.argv[1])
+got = []
+for _ in range(3):
+    cfg = problems.khi2d(n=8)[0]
+    cfg.inum = cfg.jnum = 1024
+    p = np.ones((4, 1028, 1028))
+    p[1:3], p[3] = 0.1, 2.5
+    s = Simulation(cfg)
+    s.set_state(abi.PVAR, p)
+    s.first_step()
+    s.run(2)
+    got.append(s.get(abi.PVAR))
+    s.close()
+    assert runtime.cudaSetDevice(0) == 0 and runtime.cudaDeviceReset() == 0
+assert np.isfinite(got[0]).all() and np.array_equal(got[0], got[1]) and np.array_equal(got[0], got[2])
+print("done")
+"""
+
+
+@pytest.mark.gpu
+def test_device_reset_between_grids():
+    """A program (of its own process) that resets the device once its grids are closed opens new ones: the
+    lanes, which went with the old context, are made anew."""
+    import glob
+    import os
+    import subprocess
+    import sys
+
+    import torch
+    found = glob.glob(os.path.join(os.path.dirname(os.path.dirname(torch.__file__)), "nvidia", "cuda_runtime", "lib",
+                                   "libcudart.so*")) + glob.glob("/usr/local/cuda/lib64/libcudart.so*")
+    if not found:
+        pytest.skip("no shared CUDA runtime here")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _RESET, found[0]], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "done" in r.stdout, r.stderr[-2000:]

@@ -22,10 +22,12 @@ RUNTIME = r'''
 #include <cstring>
 #include <thread>
 typedef int cudaError_t;
-typedef struct Stream { int device; } *cudaStream_t;
-typedef struct Event { int device; } *cudaEvent_t;
+typedef struct Stream { int device; unsigned long long context; } *cudaStream_t;
+typedef struct Event { int device; unsigned long long context; } *cudaEvent_t;
 enum { cudaSuccess = 0, cudaErrorMemoryAllocation = 2, cudaErrorInvalidResourceHandle = 400 };
 enum { cudaStreamNonBlocking = 1, cudaEventDisableTiming = 2, cudaMemoryTypeUnregistered = 0 };
+enum { cudaEnableDefault = 0 };
+enum cudaDriverEntryPointQueryResult { cudaDriverEntryPointSuccess };
 enum cudaMemcpyKind { cudaMemcpyHostToDevice = 1, cudaMemcpyDeviceToHost = 2 };
 enum cudaStreamCaptureMode { cudaStreamCaptureModeGlobal, cudaStreamCaptureModeThreadLocal, cudaStreamCaptureModeRelaxed };
 struct cudaPointerAttributes { int type; };
@@ -35,7 +37,10 @@ inline std::atomic<long long> piece{0};   // of the largest copy
 inline std::atomic<int> held{0};          // copies wait while it is set
 inline thread_local int device = 0;
 inline thread_local cudaStreamCaptureMode mode = cudaStreamCaptureModeGlobal;
-struct Head { size_t n; char pad[56]; };
+inline std::atomic<unsigned long long> context[32];   // of each device; a reset makes another
+inline std::atomic<long long> stale{0};                 // uses of what went with a context
+inline unsigned long long now() { return 100 * device + context[device]; }
+struct Head { size_t n; unsigned long long context; int device; char pad[44]; };
 }  // namespace fake
 inline cudaError_t cudaGetLastError() { return 0; }
 inline cudaError_t cudaSetDevice(int d) { fake::device = d; return 0; }
@@ -47,31 +52,41 @@ inline cudaError_t cudaThreadExchangeStreamCaptureMode(cudaStreamCaptureMode* m)
   return 0;
 }
 inline cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void*) { a->type = 0; return 0; }
-enum { cudaHostAllocPortable = 1 };
 inline cudaError_t cudaMallocHost(void** p, size_t n) {
   fake::Head* h = static_cast<fake::Head*>(std::malloc(sizeof(fake::Head) + n));
   h->n = n;
+  h->context = fake::now();
+  h->device = fake::device;
   *p = h + 1;
   ++fake::pins;
   fake::bytes += n;
   return 0;
 }
-inline cudaError_t cudaHostAlloc(void** p, size_t n, int) { return cudaMallocHost(p, n); }
 inline cudaError_t cudaFreeHost(void* p) {
   fake::Head* h = static_cast<fake::Head*>(p) - 1;
+  fake::stale += h->context != 100 * h->device + fake::context[h->device];
   fake::bytes -= h->n;
   ++fake::frees;
   std::free(h);
   return 0;
 }
-inline cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, int) { ++fake::streams; *s = new Stream{fake::device}; return 0; }
-inline cudaError_t cudaStreamDestroy(cudaStream_t s) { ++fake::destroyed; delete s; return 0; }
-inline cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, int) { *e = new Event{fake::device}; return 0; }
-inline cudaError_t cudaEventDestroy(cudaEvent_t e) { delete e; return 0; }
-inline cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return 0; }
-inline cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, int) { return 0; }
-inline cudaError_t cudaStreamSynchronize(cudaStream_t) { ++fake::waits; return 0; }
+inline cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, int) { ++fake::streams; *s = new Stream{fake::device, fake::now()}; return 0; }
+template <class T>
+void used(T* h) { fake::stale += h && h->context != 100 * h->device + fake::context[h->device]; }
+inline cudaError_t cudaStreamDestroy(cudaStream_t s) { used(s); ++fake::destroyed; delete s; return 0; }
+inline cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, int) { *e = new Event{fake::device, fake::now()}; return 0; }
+inline cudaError_t cudaEventDestroy(cudaEvent_t e) { used(e); delete e; return 0; }
+inline cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t) { used(e); return 0; }
+inline cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, int) { used(s); used(e); return 0; }
+inline cudaError_t cudaStreamSynchronize(cudaStream_t s) { used(s); ++fake::waits; return 0; }
+inline int context_id(void*, unsigned long long* id) { *id = fake::now(); return 0; }
+inline int context_state(int d, unsigned*, int* active) { *active = fake::context[d] % 2 == 0; return 0; }
+inline cudaError_t cudaGetDriverEntryPoint(const char* name, void** p, unsigned long long, cudaDriverEntryPointQueryResult*) {
+  *p = std::strcmp(name, "cuCtxGetId") == 0 ? reinterpret_cast<void*>(context_id) : reinterpret_cast<void*>(context_state);
+  return 0;
+}
 inline cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t stream) {
+  used(stream);
   if (stream && stream->device != fake::device) return cudaErrorInvalidResourceHandle;
   std::memcpy(d, s, n);
   ++fake::copies;
@@ -106,15 +121,17 @@ int copy(void* t, void* host, void* dev, size_t n, int to_host, int device) {
   }
 }
 void starve(int on) { starved = on; }
+// a device's context goes (odd: none yet), or another one comes
+void reset(int device) { ++fake::context[device]; }
 void hold(int on) { fake::held = on; }
 long long count(int what) {
   std::atomic<long long>* c[] = {&fake::pins, &fake::frees, &fake::bytes, &fake::streams, &fake::destroyed,
-                                 &fake::copies, &fake::waits, &fake::piece};
+                                 &fake::copies, &fake::waits, &fake::piece, &fake::stale};
   return *c[what];
 }
 }
 '''
-PINS, FREES, PINNED, STREAMS, DESTROYED, COPIES, WAITS, PIECE = range(8)
+PINS, FREES, PINNED, STREAMS, DESTROYED, COPIES, WAITS, PIECE, STALE = range(9)
 MB = 1 << 20
 
 
@@ -138,7 +155,7 @@ class _Lanes:
 
     def __init__(self, lib):
         self.L, self.t = lib, C.c_void_p(lib.make())
-        self.start = [lib.count(q) for q in range(8)]
+        self.start = [lib.count(q) for q in range(9)]
 
     def count(self, what):
         return self.L.count(what) - self.start[what]
@@ -212,15 +229,15 @@ def test_slots_grow_with_the_transfers(lib):
 
 
 def test_devices_in_turn(lib):
-    """Handles on several devices that transfer in turn: the slots are pinned once, the streams of each
-    device made once, and every piece goes through a stream of its device."""
+    """Handles on several devices that transfer in turn: the lanes of each device are made once, and
+    every piece goes through a stream of its device."""
     t = _Lanes(lib)
     t.attach()
     t.copy(2 * MB, device=0)
     lanes = t.count(STREAMS)
     for device in (0, 1, 2, 1, 0, 2):
         assert t.copy(2 * MB, device=device) == 0
-    assert t.count(PINS) == 1 and t.count(STREAMS) == 3 * lanes and t.count(DESTROYED) == 0
+    assert t.count(PINS) == 3 and t.count(STREAMS) == 3 * lanes and t.count(FREES) == t.count(DESTROYED) == 0
     for device in range(3, 20):   # more devices than have room: the driver's path
         assert t.copy(2 * MB, device=device) == 0
     assert t.count(STREAMS) <= 16 * lanes
@@ -304,3 +321,25 @@ def test_the_lanes_are_internal_to_a_library(name):
     names = subprocess.run(["nm", "-D", "--defined-only", path], check=True, capture_output=True, text=True).stdout
     assert "fgpu_create" in names
     assert not [n for n in names.splitlines() if " u " in n and "Transfer" in n]
+
+
+def test_a_context_that_was_reset(lib):
+    """A program that resets the device between two grids: nothing that went with the old context is used or
+    freed, neither by the next transfer nor when the lanes are given back."""
+    t = _Lanes(lib)
+    t.attach()
+    assert t.copy(2 * MB) == 0 and t.copy(2 * MB, device=1) == 0
+    t.detach()
+    lib.reset(0)
+    lib.reset(0)
+    t.attach()
+    assert t.copy(3 * MB) == 0 and t.count(PINS) == 3
+    t.detach()
+    lib.reset(1)      # gone, and no other one yet
+    t.attach()
+    t.detach()        # the idle handle takes the living context's lanes along
+    assert t.count(FREES) == 1 and t.count(STALE) == 0
+    lib.reset(1)
+    t.attach()
+    assert t.copy(2 * MB, device=1) == 0 and t.count(STALE) == 0
+    t.detach()
