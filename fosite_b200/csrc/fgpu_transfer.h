@@ -162,18 +162,18 @@ class Transfer {
   }
   // Driver calls: the identity of the current context (never used twice in a process), and whether a
   // device's context exists (cudaSetDevice would make one).
-  static unsigned long long current_context() {
-    static int (*const get_id)(void*, unsigned long long*) =
-        reinterpret_cast<int (*)(void*, unsigned long long*)>(driver_call("cuCtxGetId"));
+  int (*get_id_)(void*, unsigned long long*) = nullptr;
+  int (*get_state_)(int, unsigned*, int*) = nullptr;
+  unsigned long long current_context() {
+    if (!get_id_) get_id_ = reinterpret_cast<int (*)(void*, unsigned long long*)>(driver_call("cuCtxGetId"));
     unsigned long long id = 0;
-    return get_id && get_id(nullptr, &id) == 0 ? id : 0;
+    return get_id_ && get_id_(nullptr, &id) == 0 ? id : 0;
   }
-  static bool has_context(int device) {
-    static int (*const get_state)(int, unsigned*, int*) =
-        reinterpret_cast<int (*)(int, unsigned*, int*)>(driver_call("cuDevicePrimaryCtxGetState"));
+  bool has_context(int device) {
+    if (!get_state_) get_state_ = reinterpret_cast<int (*)(int, unsigned*, int*)>(driver_call("cuDevicePrimaryCtxGetState"));
     unsigned flags = 0;
     int active = 1;
-    return !get_state || get_state(device, &flags, &active) != 0 || active != 0;
+    return !get_state_ || get_state_(device, &flags, &active) != 0 || active != 0;
   }
   static void* driver_call(const char* name) {
     void* p = nullptr;
