@@ -592,8 +592,9 @@ struct Cells {
   // ip = padded i; out[0] = 2D sum or x; out[1], out[2] for 3D; out[3] the inverse
   // viscous time step of sources_viscosity.f90:532-575, sum over the directions of
   // (max wave speed + 2*kinvis/dl)/dl with kinvis = dynvis/density (0 without viscosity).
-  // WIDE: an interior cell of a stage, whose width is not 0 (one on the axis has no volume either, and
-  // no finite state after its first stage): the test costs the 3D stage kernel registers, 2% of it.
+  // WIDE: an interior cell of a stage or of the transport, whose width is not 0 (one on the axis has
+  // no volume either, and no finite state after its first stage): the test costs the 3D stage kernel
+  // registers, 2% of it.
   template <bool WIDE = false>
   static __device__ __forceinline__ void cfl_cell(const double* p, double cs, const MetricP& M, int ip, double* out) {
     double dl[3] = {M.dlx[ip], M.dly[ip], ND == 3 ? M.dlz[ip] : 1.0};

@@ -304,7 +304,7 @@ __device__ __forceinline__ void fargo_advect_body(const FargoAdvArgs& A, const i
         for (int v = 0; v < V; ++v) if (invalid_value(p[v]) || invalid_value(c[v])) flags |= 0x08;
       p[2] = p[2] - w;
       double v3[4];
-      CE::cfl_cell(p, csc, M, ip, v3);
+      CE::template cfl_cell<true>(p, csc, M, ip, v3);
       cflv = dmax(cflv, v3[0]);
       cflvis = dmax(cflvis, v3[3]);
 #pragma unroll
@@ -398,7 +398,7 @@ __device__ __forceinline__ void fargo_advect_x_body(const FargoAdvArgs& A, const
       for (int v = 0; v < V; ++v) if (invalid_value(p[v]) || invalid_value(c[v])) flags |= 0x08;
     p[1] = p[1] - w;
     double v3[4];
-    CE::cfl_cell(p, csc, M, ipd, v3);
+    CE::template cfl_cell<true>(p, csc, M, ipd, v3);
     cflv = dmax(cflv, v3[0]);
     cflvis = dmax(cflvis, v3[3]);
   }
